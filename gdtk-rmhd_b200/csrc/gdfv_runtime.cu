@@ -809,6 +809,7 @@ int do_prepare(Context* c) {
     NumParams& P = c->P;
     P.gas.R = g.R; P.gas.gamma = g.gamma; P.gas.Cv = Cv; P.gas.Cvinv = 1.0 / Cv;
     P.eps_van_albada = g.eps_van_albada;
+    P.eps_in_range = g.eps_van_albada >= 1.0e-200 && g.eps_van_albada <= 1.0e200;
     P.divB_damping_length = g.divB_damping_length;
     P.max_velocity = g.max_velocity; P.max_temp = g.max_temp; P.min_temp = g.min_temp;
     P.apply_limiter = g.apply_limiter; P.extrema_clipping = g.extrema_clipping;

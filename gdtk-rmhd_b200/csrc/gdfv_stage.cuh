@@ -196,7 +196,7 @@ __device__ __forceinline__ void decode_prim_g(double Cvinv, double gR, const dou
         double r0 = (double)__frcp_rn((float)rho);
         dinv = r0 * (2.0 - rho * r0);
     } else {
-        dinv = 1.0 / rho;
+        dinv = inverse(rho);
     }
     s.rho = rho;
     s.v[0] = U[XMOM] * dinv;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void decode_prim_g(double Cvinv, double gR, const dou
     s.u = u;
     double T = u * Cvinv;
     if (FAST) s.a = (double)sqrtf((float)(gR * T));
-    else s.a = sqrt(gR * T);
+    else s.a = square_root(gR * T);
 }
 
 template <bool FAST, bool MHD>
@@ -394,6 +394,58 @@ __device__ __forceinline__ float clip_fast(float q, float A, float B) {
     return fminf(fmaxf(q, fminf(A, B)), fmaxf(A, B));
 }
 
+// num / den of the limiter for an epsilon whose denominators quot() does not take.
+static __device__ __noinline__ double limiter_quotient(double num, double den) { return num / den; }
+// The limiter of a scalar (e4/onedinterp.d:367-371): (p + |p| + eps) / (dm^2 + dp^2 + eps), p = dm dp.
+template <class R, bool FD>
+__device__ __forceinline__ R limiter(R dm, R dp, R eps) {
+    const R num = dm * dp + rabs(dm * dp) + eps, den = dm * dm + dp * dp + eps;
+    if constexpr (FD) return quot(num, recip(den));
+    else if constexpr (sizeof(R) == 8) return limiter_quotient(num, den);
+    else return num / den;
+}
+
+// The operations of interp_l2r2_scalar in the reference's order (FD: quot for the limiter).
+template <class R, int NRS, bool MHD, int OPT, bool FD>
+__device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, const R* qm1, const R* q0, const R* qp1,
+                                              R* qm, R* qp) {
+    const R t = w[W_TOC];
+    const R aL0 = w[W_AL0], aR0 = w[W_AR0], len = w[W_LENL0], w3 = w[W_TWOL];
+    const bool lim = OPT == 1 ? true : (bool)P.apply_limiter;
+    const bool clip = OPT == 1 ? true : (bool)P.extrema_clipping;
+    const R eps = R(P.eps_van_albada);
+#pragma unroll
+    for (int s = 0; s < NRS; ++s) {
+        if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
+        R dm = (q0[s] - qm1[s]) * t;
+        R dp = (qp1[s] - q0[s]) * t;
+        R sl = R(1.0), slm = R(1.0);
+        if (lim) {
+            if (OPT == 0 && P.lmr_epsilon) {
+                // lmr/onedinterp.d:147-151: each face's epsilon is scaled by the larger of
+                // its two states, so the plus face (q0, qp1) and the minus face (qm1, q0)
+                // of the cell get separate limiter values
+                const R tiny = R(1e-12);
+                const R ep = rmax(rmax(tiny, rabs(q0[s])), rmax(tiny, rabs(qp1[s]))) * eps * t;
+                const R em = rmax(rmax(tiny, rabs(qm1[s])), rmax(tiny, rabs(q0[s]))) * eps * t;
+                sl = limiter<R, FD>(dm, dp, ep);
+                slm = limiter<R, FD>(dm, dp, em);
+            } else {
+                sl = limiter<R, FD>(dm, dp, eps);
+                slm = sl;
+            }
+        }
+        R vp = q0[s] + sl * aL0 * (dp * w3 + dm * len);
+        R vm = q0[s] - slm * aR0 * (dp * len + dm * w3);
+        if (clip) {
+            vp = clip_fast(vp, q0[s], qp1[s]);
+            vm = clip_fast(vm, qm1[s], q0[s]);
+        }
+        qp[s] = vp;
+        qm[s] = vm;
+    }
+}
+
 // One cell, one direction: both interface values of every reconstructed scalar
 // (e4/onedinterp.d:338-386 with beta = 1 and equal lengths).  qm[s]: value at
 // the cell's minus face (right state there), qp[s]: at its plus face (left state).
@@ -446,49 +498,23 @@ __device__ __forceinline__ void recon_cell(const R* w, const R* wf, const NumPar
             qm[s] = q0[s] - sl * (R1 * b + R2 * a);
         }
     } else {
-        const R t = w[W_TOC];
-        const R aL0 = w[W_AL0], aR0 = w[W_AR0], len = w[W_LENL0], w3 = w[W_TWOL];
-        const bool lim = OPT == 1 ? true : (bool)P.apply_limiter;
-        const bool clip = OPT == 1 ? true : (bool)P.extrema_clipping;
-        const R eps = R(P.eps_van_albada);
-#pragma unroll
-        for (int s = 0; s < NRS; ++s) {
-            if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
-            R dm = (q0[s] - qm1[s]) * t;
-            R dp = (qp1[s] - q0[s]) * t;
-            R sl = R(1.0), slm = R(1.0);
-            if (lim) {
-                if (OPT == 0 && P.lmr_epsilon) {
-                    // lmr/onedinterp.d:147-151: each face's epsilon is scaled by the larger of
-                    // its two states, so the plus face (q0, qp1) and the minus face (qm1, q0)
-                    // of the cell get separate limiter values
-                    const R tiny = R(1e-12);
-                    const R ep = rmax(rmax(tiny, rabs(q0[s])), rmax(tiny, rabs(qp1[s]))) * eps * t;
-                    const R em = rmax(rmax(tiny, rabs(qm1[s])), rmax(tiny, rabs(q0[s]))) * eps * t;
-                    sl = (dm * dp + rabs(dm * dp) + ep) / (dm * dm + dp * dp + ep);
-                    slm = (dm * dp + rabs(dm * dp) + em) / (dm * dm + dp * dp + em);
-                } else {
-                    sl = (dm * dp + rabs(dm * dp) + eps) / (dm * dm + dp * dp + eps);
-                    slm = sl;
-                }
+        // FP64: the scalars' limiter quotients without branches (quot), so that they run
+        // interleaved; per scalar and out of line for an epsilon out of quot's range
+        if constexpr (sizeof(R) == 8) {
+            if (P.eps_in_range) {
+                recon_cell_of<R, NRS, MHD, OPT, true>(w, P, qm1, q0, qp1, qm, qp);
+                return;
             }
-            R vp = q0[s] + sl * aL0 * (dp * w3 + dm * len);
-            R vm = q0[s] - slm * aR0 * (dp * len + dm * w3);
-            if (clip) {
-                vp = clip_fast(vp, q0[s], qp1[s]);
-                vm = clip_fast(vm, qm1[s], q0[s]);
-            }
-            qp[s] = vp;
-            qm[s] = vm;
         }
+        recon_cell_of<R, NRS, MHD, OPT, false>(w, P, qm1, q0, qp1, qm, qp);
     }
 }
 
 // recon_cell for a cell of a graded block: the weights g[GW_*] of the cell's position
 // along the direction (e4/onedinterp.d:338-386 with the lengths of cells c-1, c, c+1;
 // the two scaled differences are those of both faces of the cell, as on a uniform grid).
-template <class R, int NRS, bool MHD>
-__device__ __forceinline__ void recon_cell_graded(const double* g, const NumParams& P, const R* qm1, const R* q0,
+template <class R, int NRS, bool MHD, bool FD>
+__device__ __forceinline__ void recon_cell_graded_of(const double* g, const NumParams& P, const R* qm1, const R* q0,
                                                   const R* qp1, R* qm, R* qp) {
     const R tol = R(g[GW_TOL]), toc = R(g[GW_TOC]), a = R(g[GW_A]);
     const R twoL = R(g[GW_TWOL]), lenR0 = R(g[GW_LENR0]), lenL0 = R(g[GW_LENL0]), twoR = R(g[GW_TWOR]);
@@ -499,7 +525,7 @@ __device__ __forceinline__ void recon_cell_graded(const double* g, const NumPara
         R dm = (q0[s] - qm1[s]) * tol;
         R dp = (qp1[s] - q0[s]) * toc;
         R sl = R(1.0);
-        if (P.apply_limiter) sl = (dm * dp + rabs(dm * dp) + eps) / (dm * dm + dp * dp + eps);
+        if (P.apply_limiter) sl = limiter<R, FD>(dm, dp, eps);
         R vp = q0[s] + sl * a * (dp * twoL + dm * lenR0);
         R vm = q0[s] - sl * a * (dp * lenL0 + dm * twoR);
         if (P.extrema_clipping) {
@@ -509,6 +535,17 @@ __device__ __forceinline__ void recon_cell_graded(const double* g, const NumPara
         qp[s] = vp;
         qm[s] = vm;
     }
+}
+template <class R, int NRS, bool MHD>
+__device__ __forceinline__ void recon_cell_graded(const double* g, const NumParams& P, const R* qm1, const R* q0,
+                                                  const R* qp1, R* qm, R* qp) {
+    if constexpr (sizeof(R) == 8) {
+        if (P.eps_in_range) {
+            recon_cell_graded_of<R, NRS, MHD, true>(g, P, qm1, q0, qp1, qm, qp);
+            return;
+        }
+    }
+    recon_cell_graded_of<R, NRS, MHD, false>(g, P, qm1, q0, qp1, qm, qp);
 }
 
 // AUSMDV (e4/fluxcalc.d:477-651) for the float-flux ideal-gas variant.  The
@@ -607,6 +644,26 @@ __device__ __forceinline__ void simple_outflow_flux(const NumParams& P, const R*
     }
 }
 
+template <class R, int FLUX, bool FD>
+__device__ __forceinline__ void flux_of(const NumParams& P, const FaceState<R>& L, const FaceState<R>& Rr, R* F) {
+    if (FLUX == FLUX_AUSMDV) ausmdv<R, FD>(P, L, Rr, F);
+    else if (FLUX == FLUX_HLLC) hllc<R, FD>(P, L, Rr, F);
+    else hlle_mhd<R, FD>(P, L, Rr, F);
+}
+struct FluxVec {
+    double F[10];
+};
+template <int FLUX>
+__device__ __noinline__ FluxVec flux_out_of_range(GasParams gas, int entropy_fix, FaceState<double> L,
+                                                  FaceState<double> Rr) {
+    NumParams P{};
+    P.gas = gas;
+    P.apply_entropy_fix = entropy_fix;
+    FluxVec G;
+    flux_of<double, FLUX, false>(P, L, Rr, G.F);
+    return G;
+}
+
 // Interface flux from reconstructed left/right scalars (face-local frame)
 // plus the centre states of the two adjacent cells (prim arrays pl/pr, entries
 // il/ir, variable stride `stride`): their sound speed is kept (the rhou update
@@ -669,9 +726,26 @@ __device__ __forceinline__ void face_flux(const NumParams& P, R c_h, const R* qL
     L.a = pl[5 * stride + il];
     Rr.a = pr[5 * stride + ir];
     R F[NQ];
-    if (FLUX == FLUX_AUSMDV) ausmdv(P, L, Rr, F);
-    else if (FLUX == FLUX_HLLC) hllc(P, L, Rr, F);
-    else hlle_mhd(P, L, Rr, F);
+    if constexpr (sizeof(R) == 8) {
+        // the flux's divisors are sums and products of these; out of range (outside about
+        // 1e-30 .. 1e30) it runs with the compiler's division, out of line
+        HiRange h;
+        h.take(L.rho); h.take(Rr.rho); h.take(L.p); h.take(Rr.p); h.take(L.a); h.take(Rr.a);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            h.take_below(L.v[m]); h.take_below(Rr.v[m]);
+            if (MHD) { h.take_below(L.B[m]); h.take_below(Rr.B[m]); }
+        }
+        if (h.in_range()) {
+            flux_of<R, FLUX, true>(P, L, Rr, F);
+        } else {
+            const FluxVec G = flux_out_of_range<FLUX>(P.gas, P.apply_entropy_fix, L, Rr);
+#pragma unroll
+            for (int q = 0; q < (MHD ? 8 : 5); ++q) F[q] = G.F[q];
+        }
+    } else {
+        flux_of<R, FLUX, false>(P, L, Rr, F);
+    }
     if (MHD) {
         // fluxcalc.d:139-150; the reference adds the third term to F[xB] (:146)
         F[PSI] = R(0.0);
