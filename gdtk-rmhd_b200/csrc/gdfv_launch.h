@@ -52,6 +52,9 @@ inline int tile_rows_corrector(int precision, bool mhd) {
     return precision == 0 ? (mhd ? TJ_FP64_MHD : TJ_FP64_CORR) : (mhd ? TJ_FP32_MHD_CORR : TJ_FP32_CORR);
 }
 
+// CTAs of the stage kernels resident on one SM (their launch bounds and shared memory).
+inline int tile_ctas_per_sm(int precision, bool mhd) { return precision == 0 ? (mhd ? 1 : 2) : (mhd ? 2 : 3); }
+
 // Options under which the float-flux Euler stages run the kernel on decoded primitives
 // (gdfv_stage_prim.cuh) when the arguments carry primitive buffers (the FP64 form keeps
 // stage_kernel, which ran faster than an FP64 build of the primitive kernel): the

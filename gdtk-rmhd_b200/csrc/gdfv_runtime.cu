@@ -230,6 +230,7 @@ struct Context {
     bool prepared = false;
     std::string err;
     int device = 0;
+    int n_sm = 148;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     long long total = 0;
@@ -503,8 +504,36 @@ void fill_weights(double len, double* w) {
     w[W_TWOR] = (2.0 * lenR0 + lenR1);
 }
 
-// Tile table over all blocks: 32 x TJ columns and kchunk planes per tile (0: the
-// block's nkc up to 32).  Ordered by decreasing work (cells), so that a grid
+// Planes per tile when the configuration leaves the choice (tile_kchunk 0).  A stage's
+// time follows (planes per tile + P) x waves: a tile marches its planes one after the
+// other, its prologue costs about P planes (measured 1.5; 3 for the float Euler kernel,
+// whose planes are cheaper), and the tiles run T / slots at a time, plus about a third of
+// a wave for the uneven end.  The chunk with the least product, up to 32, is taken: the
+// old fixed chunk of 32 left most SMs idle on small blocks.  Both stages at 32^3 FP64:
+// 563 us with 32 planes a tile, 50 us with 1; 64^3 570 / 153 us (6 planes), 96x80x64 573 /
+// 281 us (12), float 128x128x64 293 / 187 us (12), Orszag-Tang 64x64x32 FP64 886 / 211 us.
+// From about 9 waves on (256^3) it stays 32.
+int default_kchunk(const Context* c, int TI, int TJ, int n_sm) {
+    if (c->cfg.dims == 2) return 1;
+    const double slots = (double)n_sm * tile_ctas_per_sm(c->cfg.precision, c->cfg.mhd);
+    const double prologue = c->cfg.precision == 1 && !c->cfg.mhd ? 3.0 : 1.5;
+    int best = 32;
+    double least = 1e300;
+    for (int kc : {32, 24, 16, 12, 8, 6, 4, 3, 2, 1}) {
+        double tiles = 0.0, deep = 0.0;
+        for (const HostBlock& hb : c->blocks) {
+            const int m = (hb.n[2] + kc - 1) / kc;
+            tiles += (double)m * ((hb.n[0] + TI - 1) / TI) * ((hb.n[1] + TJ - 1) / TJ);
+            deep = std::max(deep, (double)((hb.n[2] + m - 1) / m));
+        }
+        const double cost = (deep + prologue) * std::max(1.0, tiles / slots + 0.35);
+        if (cost < least) { least = cost; best = kc; }
+    }
+    return best;
+}
+
+// Tile table over all blocks: 32 x TJ columns and kchunk planes per tile (0:
+// default_kchunk, evened out over the chunks of each block).  Ordered by decreasing work (cells), so that a grid
 // taking tiles in order -- the hardware's CTA order, or the persistent stride --
 // starts the long tiles of uneven blocks first.
 // Tiles of TI x TJ cells (k chunks of kchunk planes) over the i strips (i0 a multiple of
@@ -512,9 +541,11 @@ void fill_weights(double len, double* w) {
 template <class Pick>
 void build_tiles_strips(Context* c, int kchunk, int TI, int TJ, Pick pick, std::vector<TileDesc>& tiles) {
     tiles.clear();
+    const int auto_kc = kchunk > 0 ? kchunk : default_kchunk(c, TI, TJ, c->n_sm);
     for (size_t b = 0; b < c->blocks.size(); ++b) {
         const HostBlock& hb = c->blocks[b];
-        int kc = kchunk > 0 ? kchunk : std::min(hb.n[2], 32);
+        const int chunks = (hb.n[2] + auto_kc - 1) / auto_kc;
+        int kc = kchunk > 0 ? kchunk : (hb.n[2] + chunks - 1) / chunks;
         if (c->cfg.dims == 2) kc = 1;
         for (int k0 = 0; k0 < hb.n[2]; k0 += kc)
             for (int j0 = 0; j0 < hb.n[1]; j0 += TJ)
@@ -825,10 +856,11 @@ int do_prepare(Context* c) {
     sp.max_attempts = g.max_attempts; sp.max_invalid_cells = g.max_invalid_cells;
     sp.nblocks = (int)c->blocks.size();
     sp.cfl_value = g.cfl_value; sp.dt_init = g.dt_init; sp.dt_max = g.dt_max;
+    CK(cudaGetDevice(&c->device));
+    CK(cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, c->device));
     // (after the options: the tables depend on which kernels run)
     build_tiles(c, g.tile_kchunk, tiles, c->n_tiles, c->n_tiles2, c->n_prim_wide, c->n_prim_narrow);
 
-    CK(cudaGetDevice(&c->device));
     if (c->device < 64 && !g_configured[c->device]) {
         CK(configure_stage_fp64());
         CK(configure_stage_fp32());
@@ -1686,9 +1718,19 @@ int autotune(Context* c) {
     for (const HostBlock& hb : c->blocks) maxk = std::max(maxk, hb.n[2]);
     std::vector<int> kcs;
     if (c->cfg.dims == 2) kcs.push_back(1);
-    else
-        for (int kc : {8, 12, 16, 24, 32, 64, 128})
-            if (kc <= maxk || kcs.empty()) kcs.push_back(kc);
+    else {
+        // chunks under 8 planes only where 8 planes a tile leave SMs without a tile, or the
+        // blocks are no deeper (their prologues cost more than the parallelism they add
+        // elsewhere: 128x128x64 FP64 510 us for both stages with 4 planes, 523 with 8;
+        // Orszag-Tang 256x256x4 FP64 276 with 4, 325 with 2)
+        double tiles8 = 0.0;
+        for (const HostBlock& hb : c->blocks)
+            tiles8 += (double)((hb.n[2] + 7) / 8) * ((hb.n[0] + 31) / 32) *
+                      ((hb.n[1] + tile_rows(c->cfg.precision, c->cfg.mhd) - 1) / tile_rows(c->cfg.precision, c->cfg.mhd));
+        const bool thin = maxk <= 8 || tiles8 < (double)c->n_sm;
+        for (int kc : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 64, 128})
+            if ((kc >= 8 || thin) && (kc <= maxk || kcs.empty())) kcs.push_back(kc);
+    }
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));

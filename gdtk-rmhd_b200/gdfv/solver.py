@@ -59,7 +59,7 @@ class Config:
         self.fixed_time_step = False
         self.n_ghost_cell_layers = 2
         self.glm_reference_indexing = True
-        self.tile_kchunk = 0          # planes per tile (0: the block's nkc up to 32)
+        self.tile_kchunk = 0          # planes per tile (0: up to 32, chosen from the block sizes)
         self.persistent = False       # True: stage kernels as a resident grid over the tile queue
         self.tile_width = 32          # float Euler kernel: tiles 32 or 16 cells wide
         self.autotune = False         # time tile shapes and launch forms on the first run
