@@ -32,20 +32,11 @@ namespace gdfv {
 namespace {
 
 constexpr int NP = 6;  // rho, v0, v1, v2, u, a
-constexpr int SRC_DONE = -1;  // a stencil source whose cotangent has been added already
 
 __device__ __forceinline__ double sgn(double x) { return x < 0.0 ? -1.0 : 1.0; }
 
-// Reciprocal for the adjoint arithmetic: a float estimate refined by two FP64
-// Newton steps (relative error ~1e-14); exact division outside the float range.
-__device__ __forceinline__ double rcp(double x) {
-    double ax = fabs(x);
-    if (!(ax > 1.0e-30 && ax < 1.0e30)) return 1.0 / x;
-    double r = (double)__frcp_rn((float)x);
-    r = r * (2.0 - x * r);
-    r = r * (2.0 - x * r);
-    return r;
-}
+// Reciprocal for the adjoint arithmetic (recip, gdfv_device.cuh: within an ulp or so, no branch).
+__device__ __forceinline__ double rcp(double x) { return recip(x).r; }
 
 // Reverse of clip_to_limits(q, A, B) (src/nm/limiters.d:41-50): routes g to q, A or B.
 __device__ __forceinline__ void clip_rev(double q, double A, double B, double g, double& gq, double& gA, double& gB) {
@@ -65,167 +56,121 @@ __device__ __forceinline__ void clip_rev(double q, double A, double B, double g,
     }
 }
 
-// l2r2 for one scalar with equal lengths (e4/onedinterp.d:357-386), forward and reverse.
-struct L2R2Rec {
-    double dLm, del, dRp, sL, sR, nL, dL, nR, dR, X, Y, qLr, qRr;
-    int eps_from;   // van_albada_variant lmr: epsilon from |q0| (1), |r0| (2) or the floor (0)
+// The l2r2 weights of one cell along a direction: both interface values of a cell come
+// from one limiter evaluation (see recon_cell and, for graded blocks, recon_cell_graded).
+struct CellWeights {
+    double tol, toc, a, twoL, lenR0, lenL0, twoR;
 };
-
-// LMR: the context may take van_albada_variant lmr (a face kernel with the rare rules)
-template <bool LMR>
-__device__ __forceinline__ void l2r2_fwd(const double* w, const NumParams& P, double q1, double q0, double r0,
-                                         double r1, double& qL, double& qR, L2R2Rec& t) {
-    t.dLm = (q0 - q1) * w[W_TOL];
-    t.del = (r0 - q0) * w[W_TOC];
-    t.dRp = (r1 - r0) * w[W_TOR];
-    t.sL = 1.0; t.sR = 1.0;
-    double eps = P.eps_van_albada;
-    t.eps_from = 0;
-    if (LMR && P.lmr_epsilon) {
-        // lmr/onedinterp.d:147-151: the face's epsilon scaled by the larger of its two
-        // states (both limiter values of the face take it), as the forward kernels form it
-        const double tiny = 1e-12, a0 = fabs(q0), a1 = fabs(r0);
-        const double m = fmax(fmax(tiny, a0), fmax(tiny, a1));
-        t.eps_from = m == tiny ? 0 : (a0 >= a1 ? 1 : 2);
-        eps = m * eps * w[W_TOC];
+template <bool RARE>
+__device__ __forceinline__ CellWeights cell_weights(const BlockDesc& B, int D, int c) {
+    if (RARE && B.graded) {
+        const double* g = B.gw[D] + (long long)(c + 1) * GW_N;
+        return CellWeights{g[GW_TOL], g[GW_TOC], g[GW_A], g[GW_TWOL], g[GW_LENR0], g[GW_LENL0], g[GW_TWOR]};
     }
-    if (P.apply_limiter) {
-        double pl = t.dLm * t.del, pr = t.del * t.dRp;
-        t.nL = pl + fabs(pl) + eps; t.dL = t.dLm * t.dLm + t.del * t.del + eps; t.sL = t.nL * rcp(t.dL);
-        t.nR = pr + fabs(pr) + eps; t.dR = t.del * t.del + t.dRp * t.dRp + eps; t.sR = t.nR * rcp(t.dR);
-    }
-    t.X = t.del * w[W_TWOL] + t.dLm * w[W_LENR0];
-    t.Y = t.dRp * w[W_LENL0] + t.del * w[W_TWOR];
-    t.qLr = q0 + t.sL * w[W_AL0] * t.X;
-    t.qRr = r0 - t.sR * w[W_AR0] * t.Y;
-    qL = t.qLr; qR = t.qRr;
-    if (P.extrema_clipping) {
-        qL = clip_to_limits(qL, q0, r0);
-        qR = clip_to_limits(qR, q0, r0);
-    }
+    const double* w = B.w[D];
+    return CellWeights{w[W_TOC], w[W_TOC], w[W_AL0], w[W_TWOL], w[W_LENR0], w[W_LENL0], w[W_TWOR]};
 }
 
-template <bool LMR>
-__device__ __forceinline__ void l2r2_rev(const double* w, const NumParams& P, double q1, double q0, double r0,
-                                         double r1, const L2R2Rec& t, double gqL, double gqR, double& g1,
-                                         double& g0, double& h0, double& h1) {
-    double gqLr = 0.0, gqRr = 0.0;
-    if (P.extrema_clipping) {
-        clip_rev(t.qLr, q0, r0, gqL, gqLr, g0, h0);
-        clip_rev(t.qRr, q0, r0, gqR, gqRr, g0, h0);
-    } else {
-        gqLr = gqL; gqRr = gqR;
-    }
-    double gdLm = 0.0, gdel = 0.0, gdRp = 0.0;
-    // qLr = q0 + sL*aL0*X
-    g0 += gqLr;
-    double gsL = gqLr * w[W_AL0] * t.X;
-    double gX = gqLr * t.sL * w[W_AL0];
-    gdel += gX * w[W_TWOL];
-    gdLm += gX * w[W_LENR0];
-    // qRr = r0 - sR*aR0*Y
-    h0 += gqRr;
-    double gsR = -gqRr * w[W_AR0] * t.Y;
-    double gY = -gqRr * t.sR * w[W_AR0];
-    gdRp += gY * w[W_LENL0];
-    gdel += gY * w[W_TWOR];
+// lmr/onedinterp.d:147-151: the epsilon of the face between states l and r (scaled by the
+// larger of the two), as the forward kernels form it; from: the side it came from (1 l,
+// 2 r, 0 the floor).
+__device__ __forceinline__ double lmr_epsilon(const NumParams& P, double toc, double l, double r, int& from) {
+    const double tiny = 1e-12, a0 = fabs(l), a1 = fabs(r);
+    const double m = fmax(fmax(tiny, a0), fmax(tiny, a1));
+    from = m == tiny ? 0 : (a0 >= a1 ? 1 : 2);
+    return m * P.eps_van_albada * toc;
+}
+
+// Both interface values of one scalar of a cell (q1, q0, q2: the cells before, at and after
+// it): qm at its minus face, qp at its plus face (e4/onedinterp.d:357-386, clipping as
+// src/nm/limiters.d:41-50).  rd: the reciprocal of the limiter's denominator, for the
+// reverse (not with lmr, whose two faces have limiters of their own).
+template <bool RARE>
+__device__ __forceinline__ void cell_recon(const NumParams& P, const CellWeights& w, double q1, double q0, double q2,
+                                           double& qm, double& qp, double& rd) {
+    const double dm = (q0 - q1) * w.tol, dp = (q2 - q0) * w.toc;
+    double sp = 1.0, sm = 1.0;
+    rd = 0.0;
     if (P.apply_limiter) {
-        // sL = nL/dL, nL = p + |p| + eps with p = dLm*del, dL = dLm^2 + del^2 + eps
-        const double idL = rcp(t.dL);
-        double gnL = gsL * idL, gdL = -gsL * t.sL * idL;
-        double pl = t.dLm * t.del;
-        double gpl = gnL * (1.0 + sgn(pl));
-        gdLm += gpl * t.del + gdL * 2.0 * t.dLm;
-        gdel += gpl * t.dLm + gdL * 2.0 * t.del;
-        const double idR = rcp(t.dR);
-        double gnR = gsR * idR, gdR = -gsR * t.sR * idR;
-        double pr = t.del * t.dRp;
-        double gpr = gnR * (1.0 + sgn(pr));
-        gdel += gpr * t.dRp + gdR * 2.0 * t.del;
-        gdRp += gpr * t.del + gdR * 2.0 * t.dRp;
-        if (LMR && t.eps_from) {   // lmr: epsilon enters nL, dL, nR and dR
-            const double geps = gnL + gdL + gnR + gdR;
-            const double d = geps * P.eps_van_albada * w[W_TOC];
-            if (t.eps_from == 1) g0 += d * sgn(q0);
-            else h0 += d * sgn(r0);
+        const double p = dm * dp, n = p + fabs(p), d = dm * dm + dp * dp;
+        if (RARE && P.lmr_epsilon) {
+            int from;
+            const double ep = lmr_epsilon(P, w.toc, q0, q2, from), em = lmr_epsilon(P, w.toc, q1, q0, from);
+            sp = (n + ep) * rcp(d + ep);
+            sm = (n + em) * rcp(d + em);
+        } else {
+            rd = rcp(d + P.eps_van_albada);
+            sp = sm = (n + P.eps_van_albada) * rd;
         }
     }
-    g0 += gdLm * w[W_TOL]; g1 -= gdLm * w[W_TOL];
-    h0 += gdel * w[W_TOC]; g0 -= gdel * w[W_TOC];
-    h1 += gdRp * w[W_TOR]; h0 -= gdRp * w[W_TOR];
+    qp = q0 + sp * w.a * (dp * w.twoL + dm * w.lenR0);
+    qm = q0 - sm * w.a * (dp * w.lenL0 + dm * w.twoR);
+    if (P.extrema_clipping) {
+        qp = clip_to_limits(qp, q0, q2);
+        qm = clip_to_limits(qm, q1, q0);
+    }
 }
 
-// l2r2 on a graded block (recon_cell_graded's arithmetic): the left state of the face is
-// cell L's plus-face value with L's weights gL[GW_*], the right state cell R's minus-face
-// value with R's weights gR (e4/onedinterp.d:338-386 with each cell's own lengths); the
-// difference across the face is scaled by L's and by R's weight separately.
-struct L2R2G {
-    double dLm, delL, delR, dRp, sL, sR, dL, dR, X, Y, qLr, qRr;
-};
-
-__device__ __forceinline__ void l2r2g_fwd(const double* gL, const double* gR, const NumParams& P, double q1,
-                                          double q0, double r0, double r1, double& qL, double& qR, L2R2G& t) {
-    t.dLm = (q0 - q1) * gL[GW_TOL];
-    t.delL = (r0 - q0) * gL[GW_TOC];
-    t.delR = (r0 - q0) * gR[GW_TOL];
-    t.dRp = (r1 - r0) * gR[GW_TOC];
-    t.sL = 1.0; t.sR = 1.0;
-    const double eps = P.eps_van_albada;
+// Reverse of cell_recon: the cotangents gp of qp and gm of qm onto the three cells (g0 added
+// to, g1 and g2 set).  Non-smooth points take the branch the values took.
+template <bool RARE>
+__device__ __forceinline__ void cell_recon_rev(const NumParams& P, const CellWeights& w, double q1, double q0, double q2,
+                                               double rd, double gp, double gm, double& g1, double& g0, double& g2) {
+    const double dm = (q0 - q1) * w.tol, dp = (q2 - q0) * w.toc;
+    const double p = dm * dp, n = p + fabs(p), d = dm * dm + dp * dp;
+    const bool lmr = RARE && P.lmr_epsilon;
+    double sp = 1.0, sm = 1.0, rp = rd, rm = rd;
+    int fp = 0, fm = 0;
     if (P.apply_limiter) {
-        const double pl = t.dLm * t.delL, pr = t.delR * t.dRp;
-        t.dL = t.dLm * t.dLm + t.delL * t.delL + eps; t.sL = (pl + fabs(pl) + eps) * rcp(t.dL);
-        t.dR = t.delR * t.delR + t.dRp * t.dRp + eps; t.sR = (pr + fabs(pr) + eps) * rcp(t.dR);
+        if (lmr) {
+            const double ep = lmr_epsilon(P, w.toc, q0, q2, fp), em = lmr_epsilon(P, w.toc, q1, q0, fm);
+            rp = rcp(d + ep);
+            rm = rcp(d + em);
+            sp = (n + ep) * rp;
+            sm = (n + em) * rm;
+        } else {
+            sp = sm = (n + P.eps_van_albada) * rd;
+        }
     }
-    t.X = t.delL * gL[GW_TWOL] + t.dLm * gL[GW_LENR0];
-    t.Y = t.dRp * gR[GW_LENL0] + t.delR * gR[GW_TWOR];
-    t.qLr = q0 + t.sL * gL[GW_A] * t.X;
-    t.qRr = r0 - t.sR * gR[GW_A] * t.Y;
-    qL = t.qLr; qR = t.qRr;
+    const double X = dp * w.twoL + dm * w.lenR0, Y = dp * w.lenL0 + dm * w.twoR;
+    g1 = g2 = 0.0;
+    double gvp = 0.0, gvm = 0.0;
     if (P.extrema_clipping) {
-        qL = clip_to_limits(qL, q0, r0);
-        qR = clip_to_limits(qR, q0, r0);
-    }
-}
-
-__device__ __forceinline__ void l2r2g_rev(const double* gL, const double* gR, const NumParams& P, double q0, double r0,
-                                          const L2R2G& t, double gqL, double gqR, double& g1, double& g0, double& h0,
-                                          double& h1) {
-    double gqLr = 0.0, gqRr = 0.0;
-    if (P.extrema_clipping) {
-        clip_rev(t.qLr, q0, r0, gqL, gqLr, g0, h0);
-        clip_rev(t.qRr, q0, r0, gqR, gqRr, g0, h0);
+        clip_rev(q0 + sp * w.a * X, q0, q2, gp, gvp, g0, g2);
+        clip_rev(q0 - sm * w.a * Y, q1, q0, gm, gvm, g1, g0);
     } else {
-        gqLr = gqL; gqRr = gqR;
+        gvp = gp;
+        gvm = gm;
     }
-    double gdLm = 0.0, gdelL = 0.0, gdelR = 0.0, gdRp = 0.0;
-    g0 += gqLr;
-    const double gsL = gqLr * gL[GW_A] * t.X;
-    const double gX = gqLr * t.sL * gL[GW_A];
-    gdelL += gX * gL[GW_TWOL];
-    gdLm += gX * gL[GW_LENR0];
-    h0 += gqRr;
-    const double gsR = -gqRr * gR[GW_A] * t.Y;
-    const double gY = -gqRr * t.sR * gR[GW_A];
-    gdRp += gY * gR[GW_LENL0];
-    gdelR += gY * gR[GW_TWOR];
+    g0 += gvp + gvm;
+    const double ap = gvp * w.a, am = gvm * w.a;
+    const double gX = ap * sp, gY = -am * sm;
+    double gdp = gX * w.twoL + gY * w.lenL0, gdm = gX * w.lenR0 + gY * w.twoR;
     if (P.apply_limiter) {
-        // s = (p + |p| + eps) / d with p the product of the two differences, d their squares + eps
-        const double idL = rcp(t.dL), idR = rcp(t.dR);
-        const double gnL = gsL * idL, gdL = -gsL * t.sL * idL;
-        const double pl = t.dLm * t.delL;
-        const double gpl = gnL * (1.0 + sgn(pl));
-        gdLm += gpl * t.delL + gdL * 2.0 * t.dLm;
-        gdelL += gpl * t.dLm + gdL * 2.0 * t.delL;
-        const double gnR = gsR * idR, gdR = -gsR * t.sR * idR;
-        const double pr = t.delR * t.dRp;
-        const double gpr = gnR * (1.0 + sgn(pr));
-        gdelR += gpr * t.dRp + gdR * 2.0 * t.delR;
-        gdRp += gpr * t.delR + gdR * 2.0 * t.dRp;
+        // s = (p + |p| + eps) / d, p = dm dp, d = dm^2 + dp^2 + eps
+        double gn, gd;
+        if (lmr) {
+            const double gnp = ap * X * rp, gnm = -am * Y * rm;
+            const double gdp_ = -gnp * sp, gdm_ = -gnm * sm;
+            gn = gnp + gnm;
+            gd = gdp_ + gdm_;
+            const double k = P.eps_van_albada * w.toc;   // the faces' epsilons enter n and d
+            const double ep = (gnp + gdp_) * k, em = (gnm + gdm_) * k;
+            if (fp == 1) g0 += ep * sgn(q0);
+            else if (fp == 2) g2 += ep * sgn(q2);
+            if (fm == 1) g1 += em * sgn(q1);
+            else if (fm == 2) g0 += em * sgn(q0);
+        } else {
+            gn = (ap * X - am * Y) * rd;
+            gd = -gn * sp;
+        }
+        const double gpp = gn * (1.0 + sgn(p));
+        gdm += gpp * dp + 2.0 * gd * dm;
+        gdp += gpp * dm + 2.0 * gd * dp;
     }
-    g0 += gdLm * gL[GW_TOL]; g1 -= gdLm * gL[GW_TOL];
-    h0 += gdelL * gL[GW_TOC]; g0 -= gdelL * gL[GW_TOC];
-    h0 += gdelR * gR[GW_TOL]; g0 -= gdelR * gR[GW_TOL];
-    h1 += gdRp * gR[GW_TOC]; h0 -= gdRp * gR[GW_TOC];
+    g0 += gdm * w.tol - gdp * w.toc;
+    g1 -= gdm * w.tol;
+    g2 += gdp * w.toc;
 }
 
 // ausmdv (e4/fluxcalc.d:477-651) forward with the quantities the reverse needs,
@@ -379,17 +324,17 @@ __device__ void hllc_vjp(const NumParams& P, const FS& L, const FS& R, const dou
     const double keL = 0.5 * (L.u * L.u + L.v * L.v + L.w * L.w);
     const double keR = 0.5 * (R.u * R.u + R.v * R.v + R.w * R.w);
     const double EL = L.r * L.e + L.r * keL, ER = R.r * R.e + R.r * keR;
-    const double srL = sqrt(L.r), srR = sqrt(R.r);
+    const double srL = root(L.r), srR = root(R.r);
     const double D = srL + srR, iD = rcp(D);
     const double uhat = (srL * L.u + srR * R.u) * iD;
     const double ghat = (srL * g + srR * g) * iD;
     const double N1 = srL * L.a * L.a + srR * R.a * R.a;
-    const double sD = sqrt(D);
-    const double T = D / sD;
+    const double sD = root(D), isD = rcp(sD);
+    const double T = D * isD;
     const double du = R.u - L.u;
     const double c2 = 0.5 * (ghat - 1.0);
     const double ahat2 = N1 * iD + c2 * T * du * du;
-    const double ahat = sqrt(ahat2);
+    const double ahat = root(ahat2);
     const bool SLfromL = fmin(L.u - L.a, uhat - ahat) == L.u - L.a;
     const double SL = fmin(L.u - L.a, uhat - ahat);
     const bool SRfromR = fmax(R.u + R.a, uhat + ahat) == R.u + R.a;
@@ -468,12 +413,12 @@ __device__ void hllc_vjp(const NumParams& P, const FS& L, const FS& R, const dou
     if (SLfromL) { gu_L += gSL; ga_L -= gSL; } else { guhat += gSL; gahat -= gSL; }
     if (SRfromR) { gu_R += gSR; ga_R += gSR; } else { guhat += gSR; gahat += gSR; }
     // ahat2 = N1 / D + c2 T du^2, T = D / sqrt(D); ahat = sqrt(ahat2)
-    const double gah2 = gahat * 0.5 / ahat;
+    const double gah2 = gahat * 0.5 * rcp(ahat);
     const double gN1 = gah2 * iD;
     double gD = -gah2 * N1 * iD * iD;
     double gsrL = gN1 * L.a * L.a, gsrR = gN1 * R.a * R.a;
     ga_L += gN1 * 2.0 * srL * L.a; ga_R += gN1 * 2.0 * srR * R.a;
-    gD += gah2 * c2 * du * du * 0.5 / sD;
+    gD += gah2 * c2 * du * du * 0.5 * isD;
     const double gdu = gah2 * c2 * T * 2.0 * du;
     gu_R += gdu; gu_L -= gdu;
     // uhat = (srL uL + srR uR) / D
@@ -481,7 +426,7 @@ __device__ void hllc_vjp(const NumParams& P, const FS& L, const FS& R, const dou
     gsrR += guhat * R.u * iD; gu_R += guhat * srR * iD;
     gD -= guhat * uhat * iD;
     gsrL += gD; gsrR += gD;
-    gr_L += gsrL * 0.5 / srL; gr_R += gsrR * 0.5 / srR;
+    gr_L += gsrL * 0.5 * rcp(srL); gr_R += gsrR * 0.5 * rcp(srR);
     gL = FS{gr_L, gp_L, gu_L, gv_L, gw_L, ge_L, ga_L};
     gR = FS{gr_R, gp_R, gu_R, gv_R, gw_R, ge_R, ga_R};
 }
@@ -538,46 +483,46 @@ __device__ void simple_flux_vjp(const NumParams& P, const double* q, int outsign
 struct FSm { double r, p, u, v, w, Bx, By, Bz, e; };
 
 struct FastSpeed {   // cf = sqrt(0.5 (alf + sqrt(alf^2 - 4 a2 ca2))) with its pieces
-    double a2, ca2, alf, X, als, cf2, cf;
+    double a2, ca2, alf, als, cf, ir;   // ir = 1 / rho
     bool live;        // SAFESQRT took the root
 };
 __device__ __forceinline__ FastSpeed fast_speed(double gam, double p, double rho, double Bx, double By, double Bz) {
     FastSpeed f;
     const double BB = Bx * Bx + By * By + Bz * Bz;
-    f.a2 = gam * p / rho;
-    f.ca2 = Bx * Bx / rho;
-    f.alf = f.a2 + BB / rho;
-    f.X = f.alf * f.alf - 4.0 * f.a2 * f.ca2;
-    f.live = fabs(f.X) > 1.0e-14;
-    f.als = f.live ? sqrt(f.X) : 0.0;
-    f.cf2 = 0.5 * (f.alf + f.als);
-    f.cf = sqrt(f.cf2);
+    f.ir = rcp(rho);
+    f.a2 = gam * p * f.ir;
+    f.ca2 = Bx * Bx * f.ir;
+    f.alf = f.a2 + BB * f.ir;
+    const double X = f.alf * f.alf - 4.0 * f.a2 * f.ca2;
+    f.live = fabs(X) > 1.0e-14;
+    f.als = f.live ? root(X) : 0.0;
+    f.cf = root(0.5 * (f.alf + f.als));
     return f;
 }
 // reverse of fast_speed: gcf into the cotangents of p, rho and B (added)
-__device__ __forceinline__ void fast_speed_rev(const FastSpeed& f, double gam, double p, double rho, double Bx,
-                                               double By, double Bz, double gcf, double& gp, double& grho,
-                                               double& gBx, double& gBy, double& gBz) {
-    const double gcf2 = gcf * 0.5 / f.cf;
-    double galf = 0.5 * gcf2, gals = 0.5 * gcf2;
+__device__ __forceinline__ void fast_speed_rev(const FastSpeed& f, double gam, double Bx, double By, double Bz,
+                                               double gcf, double& gp, double& grho, double& gBx, double& gBy,
+                                               double& gBz) {
+    const double gcf2 = gcf * 0.5 * rcp(f.cf);
+    double galf = 0.5 * gcf2;
+    const double gals = galf;
     double ga2 = 0.0, gca2 = 0.0;
     if (f.live) {
-        const double gX = gals * 0.5 / f.als;
+        const double gX = gals * 0.5 * rcp(f.als);
         galf += gX * 2.0 * f.alf;
         ga2 += -4.0 * f.ca2 * gX;
         gca2 += -4.0 * f.a2 * gX;
     }
-    const double BB = Bx * Bx + By * By + Bz * Bz;
     // alf = a2 + BB / rho
     ga2 += galf;
-    const double gBB = galf / rho;
-    grho -= galf * BB / (rho * rho);
+    const double gBB = galf * f.ir;
+    grho -= gBB * (f.alf - f.a2);
     // ca2 = Bx^2 / rho
-    double gBx2 = gca2 / rho;
-    grho -= gca2 * f.ca2 / rho;
+    double gBx2 = gca2 * f.ir;
+    grho -= gBx2 * f.ca2;
     // a2 = gam p / rho
-    gp += ga2 * gam / rho;
-    grho -= ga2 * f.a2 / rho;
+    gp += ga2 * gam * f.ir;
+    grho -= ga2 * f.a2 * f.ir;
     gBx2 += gBB;
     gBx += 2.0 * Bx * gBx2;
     gBy += 2.0 * By * gBB;
@@ -635,7 +580,7 @@ __device__ __forceinline__ void mhd_side_flux_rev(const FSm& S, const double* gf
 // YB, ZB; gL, gR receive the cotangents of the two states (added).
 __device__ void hlle_mhd_vjp(const NumParams& P, const FSm& L, const FSm& R, const double* gF, FSm& gL, FSm& gR) {
     // ---- forward
-    const double gam = (P.gas.Cv + P.gas.R) / P.gas.Cv;
+    const double gam = (P.gas.Cv + P.gas.R) * P.gas.Cvinv, igm1 = rcp(gam - 1.0);
     const double rho = 0.5 * (L.r + R.r), p = 0.5 * (L.p + R.p), u = 0.5 * (L.u + R.u);
     const double Bx = 0.5 * (L.Bx + R.Bx), By = 0.5 * (L.By + R.By), Bz = 0.5 * (L.Bz + R.Bz);
     const FastSpeed fm = fast_speed(gam, p, rho, Bx, By, Bz);
@@ -654,9 +599,9 @@ __device__ void hlle_mhd_vjp(const NumParams& P, const FSm& L, const FSm& R, con
     const double fLF[8] = {fl[0], fl[1], fl[2], fl[3], fl[4], 0.0, fl[5], fl[6]};
     const double fRF[8] = {fr[0], fr[1], fr[2], fr[3], fr[4], 0.0, fr[5], fr[6]};
     const double d[8] = {R.r - L.r, R.r * R.u - L.r * L.u, R.r * R.v - L.r * L.v, R.r * R.w - L.r * L.w,
-                         (R.p - L.p) / (gam - 1.0) + 0.5 * (R.r * uuR + BBR) - 0.5 * (L.r * uuL + BBL),
+                         (R.p - L.p) * igm1 + 0.5 * (R.r * uuR + BBR) - 0.5 * (L.r * uuL + BBL),
                          R.Bx - L.Bx, R.By - L.By, R.Bz - L.Bz};
-    const double iden = 1.0 / (brp - blm), fac1 = brp * blm;
+    const double iden = rcp(brp - blm), fac1 = brp * blm;
     // ---- reverse
     double gbrp = 0.0, gblm = 0.0, gfac1 = 0.0, giden = 0.0;
     double gfLF[8], gfRF[8], gd[8];
@@ -683,9 +628,9 @@ __device__ void hlle_mhd_vjp(const NumParams& P, const FSm& L, const FSm& R, con
     // wp = u + cf, wm = u - cf of the averages
     const double gu = gwp + gwm, gcf = gwp - gwm;
     double gp = 0.0, grho = 0.0, gBx = 0.0, gBy = 0.0, gBz = 0.0;
-    fast_speed_rev(fm, gam, p, rho, Bx, By, Bz, gcf, gp, grho, gBx, gBy, gBz);
-    fast_speed_rev(fL, gam, L.p, L.r, L.Bx, L.By, L.Bz, gcfL, gL.p, gL.r, gL.Bx, gL.By, gL.Bz);
-    fast_speed_rev(fR, gam, R.p, R.r, R.Bx, R.By, R.Bz, gcfR, gR.p, gR.r, gR.Bx, gR.By, gR.Bz);
+    fast_speed_rev(fm, gam, Bx, By, Bz, gcf, gp, grho, gBx, gBy, gBz);
+    fast_speed_rev(fL, gam, L.Bx, L.By, L.Bz, gcfL, gL.p, gL.r, gL.Bx, gL.By, gL.Bz);
+    fast_speed_rev(fR, gam, R.Bx, R.By, R.Bz, gcfR, gR.p, gR.r, gR.Bx, gR.By, gR.Bz);
     gL.r += 0.5 * grho; gR.r += 0.5 * grho;
     gL.p += 0.5 * gp; gR.p += 0.5 * gp;
     gL.u += 0.5 * gu; gR.u += 0.5 * gu;
@@ -701,7 +646,7 @@ __device__ void hlle_mhd_vjp(const NumParams& P, const FSm& L, const FSm& R, con
     gR.r += gd[1] * R.u; gR.u += gd[1] * R.r; gL.r -= gd[1] * L.u; gL.u -= gd[1] * L.r;
     gR.r += gd[2] * R.v; gR.v += gd[2] * R.r; gL.r -= gd[2] * L.v; gL.v -= gd[2] * L.r;
     gR.r += gd[3] * R.w; gR.w += gd[3] * R.r; gL.r -= gd[3] * L.w; gL.w -= gd[3] * L.r;
-    const double ig = gd[4] / (gam - 1.0);
+    const double ig = gd[4] * igm1;
     gR.p += ig; gL.p -= ig;
     gR.r += 0.5 * gd[4] * uuR; gL.r -= 0.5 * gd[4] * uuL;
     gR.u += gd[4] * R.r * R.u; gR.v += gd[4] * R.r * R.v; gR.w += gd[4] * R.r * R.w;
@@ -723,7 +668,7 @@ struct AdjArgs {
     double* gU;        // [nq][total]
     double* gInflow;   // [ninflow][6]
     const double* rot; // rotations of exchange faces with an Rmatrix (9 doubles each)
-    const long long* face_off;  // [3][nblocks+1] prefix counts of faces per direction
+    const long long* tile_off;  // [3][nblocks+1] prefix counts of line tiles per direction
     double* lam;       // [nq][total] adjoint state of a fused step (modes 1, 2)
     double* bbuf;      // [nq][total] b = dt/2 lam + dt mu (mode 1 writes, mode 2 is its W)
     double w_scale;    // W enters scaled by this
@@ -932,428 +877,446 @@ __device__ void adj_scatter_mhd(const AdjArgs& a, const Src& s, double x, double
     for (int m = 0; m < NPM; ++m) atomicAdd(&a.gP[m * a.total + g0], g[m]);
 }
 
-// Block and cell indices of face f of direction D (the face lies between cells
-// index-1 and index along D).
-template <int D>
-__device__ __forceinline__ int face_coords(const AdjArgs& a, long long f, int& i, int& j, int& k) {
-    const long long* off = a.face_off + D * (a.nblocks + 1);
-    int b = 0;
-    while (off[b + 1] <= f) ++b;
-    const BlockDesc& B = a.blocks[b];
-    // 32-bit: the host limits a block's faces of one direction to 2^31 - 1
-    const unsigned lf = (unsigned)(f - off[b]);
-    const unsigned nf0 = B.n[0] + (D == 0), nf1 = B.n[1] + (D == 1);
-    const unsigned r = lf / nf0;
-    i = (int)(lf - r * nf0);
-    k = (int)(r / nf1);
-    j = (int)(r - (unsigned)k * nf1);
-    return b;
+// ---------------------------------------------------------------- the face sweep
+// The transpose of reconstruction and flux along one direction, as tiles of cells of grid
+// lines: one thread per cell, which also takes the face on its plus side.
+//
+// What bounds it: FP64 latency and issue, not bytes.  A thread per face (the form before)
+// evaluates the limiter of each of its two cells forward, again in its reverse, and the two
+// reverses (20 limiters forward and 10 reverse a face for Euler), holds the four stencil
+// cells and their cotangents (168 registers, 12 warps per SM) and scatters all four with
+// atomics.  Per cell there is one limiter a scalar, forward once and reverse once; the
+// faces' states and the cotangents pass between neighbouring threads in shared memory, and
+// a cell's own cotangent, summed over its faces in this direction, is added once:
+//   1  primitives and W of the tile's cells into shared memory (ghosts by their rules)
+//   2  per cell: reconstruction; minus-face states to shared memory, plus-face ones kept
+//   3  per face: flux cotangent from W, reverse of the flux; the cotangent of the right
+//      state goes to the next cell
+//   4  per cell: reverse of the limiter: cotangents of the cells before, at and after it
+//   5  per cell: their sum, added to gP (atomically: the three directions and the tiles'
+//      ends meet there)
+// Along i a tile is 256 consecutive slots of the block's lines laid end to end, each with
+// its two ghosts on either side; along j and k it is 32 lines (lanes, i fastest, so global
+// accesses are coalesced) by 8 cells.  Neighbouring tiles share their end cells: each adds
+// the part of the faces it owns (255 slots, or 7 cells, of faces).
+constexpr int LINE_CTA = 256;
+constexpr int LINE_J = 8;      // cells along j or k per tile
+template <bool MHD>
+struct LineGeo {
+    static constexpr int NPr = MHD ? NPM : NP;   // primitives of a cell
+    static constexpr int NS = MHD ? 9 : 5;       // reconstructed scalars
+    static constexpr int NQ = MHD ? 10 : 5;
+    static constexpr int PAD = (LINE_J + 2) * 32;                  // cells with one halo layer on either side
+    static constexpr int O_P = 0;                                  // [NS][PAD] reconstructed primitives
+    static constexpr int O_W = O_P + NS * PAD;                     // [NQ][256] W (zero outside the block)
+    static constexpr int O_M = O_W + NQ * LINE_CTA;                // [NS][256] minus-face state, then its cotangent, then g1
+    static constexpr int O_R = O_M + NS * LINE_CTA;                // [NS][256] limiter reciprocal, then g2
+    static constexpr int O_A = O_R + NS * LINE_CTA;                // Euler: [256] sound speed, [256] its cotangent from the left face
+    static constexpr int O_IN = O_A + (MHD ? 0 : 2 * LINE_CTA);    // [8][NPr] inflow sums of the warps
+    static constexpr int O_END = O_IN + 8 * NPr;
+    static constexpr size_t bytes = sizeof(double) * (size_t)O_END;
+    // place of primitive v among the reconstructed ones (MHD never reconstructs the sound speed)
+    static __host__ __device__ constexpr int slot(int v) { return MHD && v > 5 ? v - 1 : v; }
+    static __host__ __device__ constexpr int prim(int s) { return MHD && s >= 5 ? s + 1 : s; }
+};
+
+// The state of cell (i, j, k) of block B, inside it or a ghost beyond one face.
+template <bool MHD, bool RARE>
+__device__ __noinline__ void line_ghost_load(const AdjArgs& a, const BlockDesc& B, int i, int j, int k, double* c) {
+    const Src s = adj_resolve<RARE>(a, B, i, j, k);
+    if constexpr (MHD)
+        adj_load_mhd(a, s, B.x0 + ((double)i + 0.5) * B.len[0], B.y0 + ((double)j + 0.5) * B.len[1], c);
+    else
+        adj_load<RARE>(a, s, c);
+}
+template <bool MHD, bool RARE>
+__device__ __noinline__ void line_ghost_scatter(const AdjArgs& a, const BlockDesc& B, int i, int j, int k,
+                                                const double* gc) {
+    const Src s = adj_resolve<RARE>(a, B, i, j, k);
+    if constexpr (MHD)
+        adj_scatter_mhd(a, s, B.x0 + ((double)i + 0.5) * B.len[0], B.y0 + ((double)j + 0.5) * B.len[1], gc);
+    else
+        adj_scatter<RARE>(a, s, gc);
 }
 
-// Source of stencil cell m (index -2, -1, 0, +1 along D from the face).  A face
-// whose four stencil cells lie inside its block (the other two indices always do)
-// takes them directly; the boundary rules apply to the others.
-template <int D, bool RARE>
-__device__ __forceinline__ Src stencil_src(const AdjArgs& a, const BlockDesc& B, int i, int j, int k, int m) {
-    const int idxD = D == 0 ? i : (D == 1 ? j : k);
-    if (idxD >= 2 && idxD + 1 < B.n[D]) {
-        const int sD = D == 0 ? 1 : (D == 1 ? B.n[0] : B.n[0] * B.n[1]);
-        const int c = i + B.n[0] * (j + B.n[1] * k) + (m - 2) * sD;
-        return Src{&B, (long long)c, -1, SRC_CELL, D, 0};
-    }
-    return adj_resolve<RARE>(a, B, i - (D == 0 ? 2 - m : 0), j - (D == 1 ? 2 - m : 0), k - (D == 2 ? 2 - m : 0));
-}
-
-// The reverse sweep of face f of direction D: cotangents gc[m] of the stencil
-// cells (added to), the kind of each stencil source and the inflow state the
-// stencil reaches (if any).  Only these small records stay live: the sources
-// themselves are resolved again when the cotangents are scattered.
-// rowid identifies the line of faces (block and the two other indices).
-template <int D, int FLUX, bool RARE>
-__device__ __forceinline__ void face_vjp(const AdjArgs& a, int b, int i, int j, int k, int* kind, int& inflow,
-                                         double (*gc)[NP], long long& rowid) {
-    const BlockDesc& B = a.blocks[b];
-    rowid = (long long)b * 0x100000000ll + (D == 0 ? (long long)j + (long long)B.n[1] * k : (long long)i);
-    double c[4][NP];
-    for (int m = 0; m < 4; ++m) {
-        const Src sm = stencil_src<D, RARE>(a, B, i, j, k, m);
-        kind[m] = sm.kind;
-        if (sm.kind == SRC_INFLOW) inflow = sm.inflow;
-        adj_load<RARE>(a, sm, c[m]);
-    }
-    // cotangent of the face flux: F enters R_right with +A/V and R_left with -A/V
-    const double AV = B.area[D] * B.vol_inv * a.w_scale;
-    const int nD = B.n[D];
-    const int idxD = D == 0 ? i : (D == 1 ? j : k);
-    const bool leftIn = idxD - 1 >= 0, rightIn = idxD < nD;
-    const long long gl = B.offset + (long long)(i - (D == 0)) + (long long)B.n[0] * ((long long)(j - (D == 1)) + (long long)B.n[1] * (k - (D == 2)));
-    const long long gr = B.offset + (long long)i + (long long)B.n[0] * ((long long)j + (long long)B.n[1] * k);
-    double AVr = AV, AVl = AV;
-    bool graded = false;
-    const double* gwL = nullptr;
-    const double* gwR = nullptr;
-    if constexpr (RARE) {
-        if (B.graded) {
-            // graded block: the face's area from the lengths of its cells across it, each
-            // side's own volume (cell lengths glen[d][c + 2], weights of cells -1 .. n)
-            graded = true;
-            const int ic[3] = {i, j, k};
-            double Lr[3], Ll[3];
-            for (int d = 0; d < 3; ++d) {
-                Lr[d] = B.glen[d][ic[d] + 2];
-                Ll[d] = B.glen[d][ic[d] - (d == D) + 2];
-            }
-            const bool threeD = a.P.dims == 3;
-            const double Af = threeD ? (D == 0 ? Lr[1] * Lr[2] : (D == 1 ? Lr[2] * Lr[0] : Lr[0] * Lr[1]))
-                                     : (D == 0 ? Lr[1] : Lr[0]);
-            const double Vr = threeD ? Lr[0] * Lr[1] * Lr[2] : Lr[0] * Lr[1];
-            const double Vl = threeD ? Ll[0] * Ll[1] * Ll[2] : Ll[0] * Ll[1];
-            AVr = Af / Vr * a.w_scale;
-            AVl = Af / Vl * a.w_scale;
-            gwL = B.gw[D] + (long long)idxD * GW_N;
-            gwR = gwL + GW_N;
-        }
-    }
-    double gFg[5];
-    for (int q = 0; q < 5; ++q) {
-        double wr = rightIn ? a.W[q * a.total + gr] : 0.0;
-        double wl = leftIn ? a.W[q * a.total + gl] : 0.0;
-        gFg[q] = AVr * wr - AVl * wl;
-    }
-    if constexpr (RARE) {
-        // OutFlowBC_SimpleFlux (boundary_flux_effect.d:504-645): the boundary face's flux is
-        // the interior cell's outflow flux, or only its pressure on a closed face
-        const int bface = idxD == 0 ? 2 * D : (idxD == nD ? 2 * D + 1 : -1);
-        if (bface >= 0 && B.bc_type[bface] == BC_SIMPLE_FLUX) {
-            const int in = (bface & 1) ? 1 : 2;   // the interior cell: left of a plus face
-            simple_flux_vjp<D>(a.P, c[in], (bface & 1) ? 1 : -1, gFg, gc[in]);
-            return;
-        }
-    }
-    constexpr int ax0 = D, ax1 = (D + 1) % 3, ax2 = (D + 2) % 3;
-    double gF[5] = {gFg[MASS], gFg[XMOM + ax0], gFg[XMOM + ax1], gFg[XMOM + ax2], gFg[TOTENERGY]};
-    // ---- forward reconstruction (local-frame scalars: vn, vt1, vt2, rho, u)
-    const double* w = B.w[D];
-    const NumParams& P = a.P;
-    const int pv[5] = {1 + ax0, 1 + ax1, 1 + ax2, 0, 4};
-    double qL[5], qR[5];
-    for (int sc = 0; sc < 5; ++sc) {
-        if (RARE && graded) {
-            L2R2G rg;
-            l2r2g_fwd(gwL, gwR, P, c[0][pv[sc]], c[1][pv[sc]], c[2][pv[sc]], c[3][pv[sc]], qL[sc], qR[sc], rg);
-            continue;
-        }
-        L2R2Rec rec;  // recomputed in the reverse sweep rather than kept live
-        l2r2_fwd<RARE>(w, P, c[0][pv[sc]], c[1][pv[sc]], c[2][pv[sc]], c[3][pv[sc]], qL[sc], qR[sc], rec);
-    }
+// Reverse of the flux of one face for Euler: left and right states in scalar order (normal
+// and tangential velocity, rho, u) with the sound speeds, gF in the face's frame; gl, gr
+// receive the cotangents in the same order, gaL, gaR those of the sound speeds.
+template <int FLUX>
+__device__ __forceinline__ void euler_face_rev(const NumParams& P, const double* l, double aL, const double* r, double aR,
+                                               const double* gF, double* gl, double& gaL, double* gr, double& gaR) {
     const double Rg = P.gas.R, Cvinv = P.gas.Cvinv;
-    bool badL = qL[4] <= 0.0 || qL[3] <= 0.0, badR = qR[4] <= 0.0 || qR[3] <= 0.0;
-    FS L, Rs;
-    if (badL) L = FS{c[1][0], c[1][0] * Rg * (c[1][4] * Cvinv), c[1][pv[0]], c[1][pv[1]], c[1][pv[2]], c[1][4], c[1][5]};
-    else L = FS{qL[3], qL[3] * Rg * (qL[4] * Cvinv), qL[0], qL[1], qL[2], qL[4], c[1][5]};
-    if (badR) Rs = FS{c[2][0], c[2][0] * Rg * (c[2][4] * Cvinv), c[2][pv[0]], c[2][pv[1]], c[2][pv[2]], c[2][4], c[2][5]};
-    else Rs = FS{qR[3], qR[3] * Rg * (qR[4] * Cvinv), qR[0], qR[1], qR[2], qR[4], c[2][5]};
-    // ---- reverse
+    const FS L{l[3], l[3] * Rg * (l[4] * Cvinv), l[0], l[1], l[2], l[4], aL};
+    const FS R{r[3], r[3] * Rg * (r[4] * Cvinv), r[0], r[1], r[2], r[4], aR};
     FS gL, gR;
-    if constexpr (FLUX == FLUX_HLLC) hllc_vjp(P, L, Rs, gF, gL, gR);
-    else ausmdv_vjp(P, L, Rs, gF, gL, gR);
-    gc[1][5] += gL.a;
-    gc[2][5] += gR.a;
-    double gqL[5] = {0, 0, 0, 0, 0}, gqR[5] = {0, 0, 0, 0, 0};
+    if constexpr (FLUX == FLUX_HLLC) hllc_vjp(P, L, R, gF, gL, gR);
+    else ausmdv_vjp(P, L, R, gF, gL, gR);
     // p = rho R (u Cvinv)
-    if (badL) {
-        gc[1][0] += gL.r + gL.p * Rg * (c[1][4] * Cvinv);
-        gc[1][4] += gL.e + gL.p * c[1][0] * Rg * Cvinv;
-        gc[1][pv[0]] += gL.u; gc[1][pv[1]] += gL.v; gc[1][pv[2]] += gL.w;
-    } else {
-        gqL[3] += gL.r + gL.p * Rg * (qL[4] * Cvinv);
-        gqL[4] += gL.e + gL.p * qL[3] * Rg * Cvinv;
-        gqL[0] += gL.u; gqL[1] += gL.v; gqL[2] += gL.w;
-    }
-    if (badR) {
-        gc[2][0] += gR.r + gR.p * Rg * (c[2][4] * Cvinv);
-        gc[2][4] += gR.e + gR.p * c[2][0] * Rg * Cvinv;
-        gc[2][pv[0]] += gR.u; gc[2][pv[1]] += gR.v; gc[2][pv[2]] += gR.w;
-    } else {
-        gqR[3] += gR.r + gR.p * Rg * (qR[4] * Cvinv);
-        gqR[4] += gR.e + gR.p * qR[3] * Rg * Cvinv;
-        gqR[0] += gR.u; gqR[1] += gR.v; gqR[2] += gR.w;
-    }
-    for (int sc = 0; sc < 5; ++sc) {
-        const int v = pv[sc];
-        if (RARE && graded) {
-            L2R2G rg;
-            double ql, qr;
-            l2r2g_fwd(gwL, gwR, P, c[0][v], c[1][v], c[2][v], c[3][v], ql, qr, rg);
-            l2r2g_rev(gwL, gwR, P, c[1][v], c[2][v], rg, gqL[sc], gqR[sc], gc[0][v], gc[1][v], gc[2][v], gc[3][v]);
-            continue;
-        }
-        L2R2Rec rec;
-        double ql, qr;
-        l2r2_fwd<RARE>(w, P, c[0][v], c[1][v], c[2][v], c[3][v], ql, qr, rec);
-        l2r2_rev<RARE>(w, P, c[0][v], c[1][v], c[2][v], c[3][v], rec, gqL[sc], gqR[sc], gc[0][v], gc[1][v], gc[2][v],
-                 gc[3][v]);
-    }
+    gl[0] = gL.u; gl[1] = gL.v; gl[2] = gL.w;
+    gl[3] = gL.r + gL.p * Rg * (l[4] * Cvinv);
+    gl[4] = gL.e + gL.p * l[3] * Rg * Cvinv;
+    gaL = gL.a;
+    gr[0] = gR.u; gr[1] = gR.v; gr[2] = gR.w;
+    gr[3] = gR.r + gR.p * Rg * (r[4] * Cvinv);
+    gr[4] = gR.e + gR.p * r[3] * Rg * Cvinv;
+    gaR = gR.a;
 }
 
-// Face f of direction D, one thread.  Along i (D = 0) the four faces whose
-// stencils share a cell are neighbouring lanes of one warp: their contributions
-// to that cell are summed with shuffles first, and one lane adds the sum
-// (same-address atomics from one warp would serialise).
-#ifndef GDFV_ADJ_MINB
-#define GDFV_ADJ_MINB 3
-#endif
-template <int D, int FLUX, bool RARE>
-__device__ __forceinline__ void face_thread(const AdjArgs& a, long long f) {
-    const long long* off = a.face_off + D * (a.nblocks + 1);
-    const bool act = f < off[a.nblocks];
-    int kind[4] = {SRC_DONE, SRC_DONE, SRC_DONE, SRC_DONE};
-    int inflow = -1;
-    double gc[4][NP];
-    for (int m = 0; m < 4; ++m)
-        for (int q = 0; q < NP; ++q) gc[m][q] = 0.0;
-    long long rowid = -1 - (long long)threadIdx.x;   // distinct for inactive lanes
-    int b = 0, i = 0, j = 0, k = 0;
-    if (act) {
-        b = face_coords<D>(a, f, i, j, k);
-        face_vjp<D, FLUX, RARE>(a, b, i, j, k, kind, inflow, gc, rowid);
-    }
-    if (D == 0) {
-        const unsigned full = 0xffffffffu;
-        const int lane = threadIdx.x & 31;
-        // source lane l + d holds the contribution of its stencil cell m to the
-        // cell of lane l (its own stencil cell 2): m = 0 at d = 2, m = 1 at d = 1, m = 3 at d = -1
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const int m = t == 0 ? 0 : (t == 1 ? 1 : 3);
-            const int d = t == 0 ? 2 : (t == 1 ? 1 : -1);
-            const bool mine = act && kind[m] == SRC_CELL;
-            const int from = lane + d, to = lane - d;
-            const long long row_from = __shfl_sync(full, rowid, from & 31);
-            const int ok_from = __shfl_sync(full, (int)mine, from & 31);
-            const long long row_to = __shfl_sync(full, rowid, to & 31);
-            const bool recv = from >= 0 && from < 32 && act && ok_from && row_from == rowid;
-            const bool sent = to >= 0 && to < 32 && mine && row_to == rowid;
-#pragma unroll
-            for (int q = 0; q < NP; ++q) {
-                const double v = __shfl_sync(full, gc[m][q], from & 31);
-                if (recv) gc[2][q] += v;
-                if (sent) gc[m][q] = 0.0;
-            }
-            if (sent) kind[m] = SRC_DONE;   // nothing left to scatter for this source
-        }
-    }
-    // Inflow ghost states are shared by every face along an inflow boundary: sum the
-    // warp's cotangents per inflow state (a face's stencil crosses at most one
-    // boundary face, so a lane carries at most one state), one atomic per state.
-    {
-        const unsigned full = 0xffffffffu;
-        int key = -1;
-        double vin[NP];
-#pragma unroll
-        for (int q = 0; q < NP; ++q) vin[q] = 0.0;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            if (act && kind[m] == SRC_INFLOW) {
-                key = inflow;
-#pragma unroll
-                for (int q = 0; q < NP; ++q) vin[q] += gc[m][q];
-                kind[m] = SRC_DONE;
-            }
-        }
-        if (__ballot_sync(full, key >= 0)) {
-            const unsigned grp = __match_any_sync(full, key);
-            const int lane = threadIdx.x & 31;
-#pragma unroll
-            for (int q = 0; q < NP; ++q) {
-                double acc = 0.0;
-                for (int src = 0; src < 32; ++src) {
-                    const double v = __shfl_sync(full, vin[q], src);
-                    if ((grp >> src) & 1u) acc += v;
-                }
-                vin[q] = acc;
-            }
-            if (key >= 0 && lane == __ffs(grp) - 1)
-                for (int q = 0; q < NP; ++q) atomicAdd(&a.gInflow[key * NP + q], vin[q]);
-        }
-    }
-    if (!act) return;
-    const BlockDesc& B = a.blocks[b];
-    for (int m = 0; m < 4; ++m)
-        if (kind[m] >= 0) adj_scatter<RARE>(a, stencil_src<D, RARE>(a, B, i, j, k, m), gc[m]);
-}
-
-// All faces of the three directions in one launch: CTAs [0, nb0) take the i faces,
-// [nb0, nb0 + nb1) the j faces, the rest the k faces (128 faces per CTA).
-constexpr int FACE_CTA = 128;
-template <int FLUX, bool RARE>
-__global__ void __launch_bounds__(FACE_CTA, GDFV_ADJ_MINB) adj_faces_kernel(AdjArgs a, unsigned nb0, unsigned nb1) {
-    const unsigned bid = blockIdx.x;
-    if (bid < nb0) face_thread<0, FLUX, RARE>(a, (long long)bid * FACE_CTA + threadIdx.x);
-    else if (bid < nb0 + nb1) face_thread<1, FLUX, RARE>(a, (long long)(bid - nb0) * FACE_CTA + threadIdx.x);
-    else face_thread<2, FLUX, RARE>(a, (long long)(bid - nb0 - nb1) * FACE_CTA + threadIdx.x);
-}
-
-// The reverse sweep of MHD face f of direction D (face_flux with hlle_mhd and the GLM
-// terms, e4/fluxcalc.d:54-187, :1608-1780): cotangents of the four stencil cells'
-// primitives, scattered through the ghost rules.  The limiter's arithmetic is the Euler
-// path's; psi is reconstructed only with divergence cleaning (a copy of the cell's
-// otherwise); c_h is the residual's, frozen.
-// Slot of primitive v in a face thread's shared-memory copy of its stencil: the sound
-// speed (5) is never reconstructed, so the nine others are kept.
-__device__ __forceinline__ constexpr int SL(int v) { return v < 5 ? v : v - 1; }
-template <int D, bool RARE>
-__device__ void face_mhd(const AdjArgs& a, long long f, double* smt) {
-    const long long* off = a.face_off + D * (a.nblocks + 1);
-    if (f >= off[a.nblocks]) return;
-    int i = 0, j = 0, k = 0;
-    const int b = face_coords<D>(a, f, i, j, k);
-    const BlockDesc& B = a.blocks[b];
+// The same for MHD: scalars with the face-frame B and psi after them; gF in the order of
+// the conserved quantities (face frame), psi and divB included.  F[divB] = (BxR - BxL)/2 and
+// the GLM terms (fluxcalc.d:139-150, with the reference's third term added to F[xB] under
+// glm_reference_indexing) with c_h held fixed, then hlle.
+__device__ __forceinline__ void mhd_face_rev(const AdjArgs& a, const double* l, const double* r, const double* gF,
+                                             double* gl, double* gr) {
     const NumParams& P = a.P;
-    Src src[4];
-    double xs[4], ys[4];
-    // the stencil's primitives and their cotangents in this thread's shared-memory slot
-    double (*c)[9] = reinterpret_cast<double (*)[9]>(smt);
-    double (*gc)[9] = reinterpret_cast<double (*)[9]>(smt + 4 * 9);
-    for (int m = 0; m < 4; ++m) {
-        src[m] = stencil_src<D, RARE>(a, B, i, j, k, m);
-        const int ci = i - (D == 0 ? 2 - m : 0), cj = j - (D == 1 ? 2 - m : 0);
-        xs[m] = B.x0 + ((double)ci + 0.5) * B.len[0];
-        ys[m] = B.y0 + ((double)cj + 0.5) * B.len[1];
-        double t[NPM];
-        adj_load_mhd(a, src[m], xs[m], ys[m], t);
-#pragma unroll
-        for (int v = 0; v < NPM; ++v) if (v != 5) c[m][SL(v)] = t[v];
-    }
-    const double AV = B.area[D] * B.vol_inv * a.w_scale;
-    const int nD = B.n[D];
-    const int idxD = D == 0 ? i : (D == 1 ? j : k);
-    const bool leftIn = idxD - 1 >= 0, rightIn = idxD < nD;
-    const long long gl = B.offset + (long long)(i - (D == 0)) +
-                         (long long)B.n[0] * ((long long)(j - (D == 1)) + (long long)B.n[1] * (k - (D == 2)));
-    const long long gr = B.offset + (long long)i + (long long)B.n[0] * ((long long)j + (long long)B.n[1] * k);
-    double gFg[10];
-    for (int q = 0; q < 10; ++q) {
-        const double wr = rightIn ? a.W[q * a.total + gr] : 0.0;
-        const double wl = leftIn ? a.W[q * a.total + gl] : 0.0;
-        gFg[q] = AV * (wr - wl);
-    }
-    constexpr int ax0 = D, ax1 = (D + 1) % 3, ax2 = (D + 2) % 3;
-    double gF[10];
-    gF[MASS] = gFg[MASS]; gF[TOTENERGY] = gFg[TOTENERGY]; gF[PSI] = gFg[PSI]; gF[DIVB] = gFg[DIVB];
-    gF[XMOM] = gFg[XMOM + ax0]; gF[YMOM] = gFg[XMOM + ax1]; gF[ZMOM] = gFg[XMOM + ax2];
-    gF[XB] = gFg[XB + ax0]; gF[YB] = gFg[XB + ax1]; gF[ZB] = gFg[XB + ax2];
-    // ---- forward reconstruction: face-frame v, rho, u, face-frame B, psi
-    const double* w = B.w[D];
-    const int pv[9] = {1 + ax0, 1 + ax1, 1 + ax2, 0, 4, 6 + ax0, 6 + ax1, 6 + ax2, 9};
-    const bool clean = P.divergence_cleaning;
-    double qL[9], qR[9];
-    for (int sc = 0; sc < 9; ++sc) {
-        if (sc == 8 && !clean) { qL[8] = c[1][SL(9)]; qR[8] = c[2][SL(9)]; continue; }
-        L2R2Rec rec;
-        l2r2_fwd<true>(w, P, c[0][SL(pv[sc])], c[1][SL(pv[sc])], c[2][SL(pv[sc])], c[3][SL(pv[sc])], qL[sc], qR[sc], rec);
-    }
     const double Rg = P.gas.R, Cvinv = P.gas.Cvinv;
-    const bool badL = qL[4] <= 0.0 || qL[3] <= 0.0, badR = qR[4] <= 0.0 || qR[3] <= 0.0;
-    auto state = [&](bool bad, const double* q, const double* cell, FSm& S, double& psi) {
-        if (bad) {   // e4/onedinterp.d:44-74: the cell-centre state
-            S = FSm{cell[SL(0)], cell[SL(0)] * Rg * (cell[SL(4)] * Cvinv), cell[SL(pv[0])], cell[SL(pv[1])], cell[SL(pv[2])],
-                    cell[SL(pv[5])], cell[SL(pv[6])], cell[SL(pv[7])], cell[SL(4)]};
-            psi = cell[SL(9)];
-        } else {
-            S = FSm{q[3], q[3] * Rg * (q[4] * Cvinv), q[0], q[1], q[2], q[5], q[6], q[7], q[4]};
-            psi = q[8];
-        }
-    };
-    FSm L, R;
-    double psiL, psiR;
-    state(badL, qL, c[1], L, psiL);
-    state(badR, qR, c[2], R, psiR);
-    // ---- reverse: F[divB] = (BxR - BxL)/2 and the GLM terms (fluxcalc.d:139-150, with the
-    // reference's third term added to F[xB] under glm_reference_indexing)
+    const FSm L{l[3], l[3] * Rg * (l[4] * Cvinv), l[0], l[1], l[2], l[5], l[6], l[7], l[4]};
+    const FSm R{r[3], r[3] * Rg * (r[4] * Cvinv), r[0], r[1], r[2], r[5], r[6], r[7], r[4]};
     FSm gL{}, gR{};
-    double gpsiL = 0.0, gpsiR = 0.0;
+    gl[8] = gr[8] = 0.0;
     gR.Bx += 0.5 * gF[DIVB]; gL.Bx -= 0.5 * gF[DIVB];
-    if (clean) {
+    if (P.divergence_cleaning) {
         const double ch = a.chd ? a.chd[0] : a.c_h;
         const double gt3 = P.glm_reference_indexing ? gF[XB] : gF[ZB];
         const double gpa = gF[XB] + gF[YB] + gt3;
         gR.Bx -= 0.5 * ch * gF[XB]; gL.Bx += 0.5 * ch * gF[XB];
         gR.By -= 0.5 * ch * gF[YB]; gL.By += 0.5 * ch * gF[YB];
         gR.Bz -= 0.5 * ch * gt3; gL.Bz += 0.5 * ch * gt3;
-        gpsiL += 0.5 * gpa; gpsiR += 0.5 * gpa;
+        gl[8] += 0.5 * gpa; gr[8] += 0.5 * gpa;
         const double gps = gF[PSI] * ch * ch;
         gL.Bx += 0.5 * gps; gR.Bx += 0.5 * gps;
-        gpsiR -= gps / (2.0 * ch); gpsiL += gps / (2.0 * ch);
+        gr[8] -= 0.5 * gF[PSI] * ch; gl[8] += 0.5 * gF[PSI] * ch;   // gps / (2 c_h)
     }
-    const double gF8[8] = {gF[MASS], gF[XMOM], gF[YMOM], gF[ZMOM], gF[TOTENERGY], gF[XB], gF[YB], gF[ZB]};
-    hlle_mhd_vjp(P, L, R, gF8, gL, gR);
-    for (int m = 0; m < 4; ++m)
-        for (int q = 0; q < 9; ++q) gc[m][q] = 0.0;
-    double gqL[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, gqR[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    auto back = [&](bool bad, const FSm& S, const FSm& gS, double gpsi, double* gq, double* gcell) {
-        // p = rho R (u Cvinv)
-        const double gr_ = gS.r + gS.p * Rg * (S.e * Cvinv), ge_ = gS.e + gS.p * S.r * Rg * Cvinv;
-        if (bad) {
-            gcell[SL(0)] += gr_; gcell[SL(4)] += ge_;
-            gcell[SL(pv[0])] += gS.u; gcell[SL(pv[1])] += gS.v; gcell[SL(pv[2])] += gS.w;
-            gcell[SL(pv[5])] += gS.Bx; gcell[SL(pv[6])] += gS.By; gcell[SL(pv[7])] += gS.Bz; gcell[SL(9)] += gpsi;
-        } else {
-            gq[3] += gr_; gq[4] += ge_;
-            gq[0] += gS.u; gq[1] += gS.v; gq[2] += gS.w;
-            gq[5] += gS.Bx; gq[6] += gS.By; gq[7] += gS.Bz; gq[8] += gpsi;
-        }
+    hlle_mhd_vjp(P, L, R, gF, gL, gR);
+    auto back = [&](const FSm& S, const FSm& gS, double* g) {
+        g[0] = gS.u; g[1] = gS.v; g[2] = gS.w;
+        g[3] = gS.r + gS.p * Rg * (S.e * Cvinv);   // p = rho R (u Cvinv)
+        g[4] = gS.e + gS.p * S.r * Rg * Cvinv;
+        g[5] = gS.Bx; g[6] = gS.By; g[7] = gS.Bz;
     };
-    back(badL, L, gL, gpsiL, gqL, gc[1]);
-    back(badR, R, gR, gpsiR, gqR, gc[2]);
-    for (int sc = 0; sc < 9; ++sc) {
-        const int v = pv[sc];
-        if (sc == 8 && !clean) { gc[1][SL(9)] += gqL[8]; gc[2][SL(9)] += gqR[8]; continue; }
-        L2R2Rec rec;
-        double ql, qr;
-        l2r2_fwd<true>(w, P, c[0][SL(v)], c[1][SL(v)], c[2][SL(v)], c[3][SL(v)], ql, qr, rec);
-        l2r2_rev<true>(w, P, c[0][SL(v)], c[1][SL(v)], c[2][SL(v)], c[3][SL(v)], rec, gqL[sc], gqR[sc], gc[0][SL(v)], gc[1][SL(v)], gc[2][SL(v)],
-                       gc[3][SL(v)]);
+    back(L, gL, gl);
+    back(R, gR, gr);
+}
+
+template <int D, bool MHD, int FLUX, bool RARE>
+__device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, double* sm) {
+    using G = LineGeo<MHD>;
+    constexpr int NS = G::NS, NQ = G::NQ, NPr = G::NPr, T = LINE_CTA, PAD = G::PAD;
+    constexpr int ax0 = D, ax1 = (D + 1) % 3, ax2 = (D + 2) % 3;
+    constexpr int step = D == 0 ? 1 : 32;   // to the next cell along D, in shared memory
+    double* SP = sm + G::O_P;
+    double* SW = sm + G::O_W;
+    double* SM = sm + G::O_M;
+    double* SR = sm + G::O_R;
+    double* SA = sm + G::O_A;
+    double* SIN = sm + G::O_IN;
+    const NumParams& P = a.P;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // place (prim slot) of scalar s: face-frame velocity, rho, u, face-frame B, psi
+    constexpr int pv[9] = {1 + ax0, 1 + ax1, 1 + ax2, 0, 4, G::slot(6 + ax0), G::slot(6 + ax1), G::slot(6 + ax2), 8};
+
+    const long long* off = a.tile_off + D * (a.nblocks + 1);
+    int b = 0;
+    while (off[b + 1] <= (long long)tile) ++b;
+    const BlockDesc& B = a.blocks[b];
+    const unsigned lt = (unsigned)((long long)tile - off[b]);
+    const int n0 = B.n[0], n1 = B.n[1], nD = B.n[D];
+    // this thread's cell: line l, index c along D (-2 .. nD + 1)
+    int c, i, j, k;
+    bool valid, first, last;   // first, last: the ends of the tile along D
+    if (D == 0) {
+        const unsigned long long x = (unsigned long long)lt * (T - 1) + (unsigned)tid;
+        valid = x < (unsigned long long)(n0 + 4) * ((unsigned long long)n1 * B.n[2]);
+        const unsigned xs = valid ? (unsigned)x : 0u, l = xs / (unsigned)(n0 + 4);
+        c = (int)(xs - l * (unsigned)(n0 + 4)) - 2;
+        i = c;
+        k = (int)(l / (unsigned)n1);
+        j = (int)(l - (unsigned)k * (unsigned)n1);
+        first = tid == 0;
+        last = tid == T - 1;
+    } else {
+        const unsigned lines = (unsigned)n0 * (unsigned)(D == 1 ? B.n[2] : n1), groups = (lines + 31) / 32;
+        const unsigned m = lt / groups, l0 = (lt - m * groups) * 32 + lane, l = l0 < lines ? l0 : 0u;
+        c = (int)m * (LINE_J - 1) - 1 + warp;
+        valid = l0 < lines && c <= nD + 1;
+        const int q = (int)(l / (unsigned)n0);
+        i = (int)(l - (unsigned)q * (unsigned)n0);
+        j = D == 1 ? c : q;
+        k = D == 1 ? q : c;
+        first = warp == 0;
+        last = warp == LINE_J - 1;
     }
-    for (int m = 0; m < 4; ++m) {
-        double t[NPM];
+    const bool inside = valid && c >= 0 && c < nD;
+    const bool active = valid && c >= -1 && c <= nD;          // cells with a face of the block
+    const bool has_face = active && c < nD && !last;          // its plus face, when the tile owns it
+    const bool has_left = active && c >= 0 && !first;         // its minus face is the tile's too
+    const int pi = D == 0 ? tid + 1 : tid + 32;               // own cell in the padded arrays
+    const int sD = D == 0 ? 1 : (D == 1 ? n0 : n0 * n1);
+    const long long g = B.offset + (long long)(unsigned)(inside ? i + n0 * (j + n1 * k) : 0);
+    const bool ends = active && (first || last);              // the tile's end cells also handle the next cell
+
+    // ---------------- 1: primitives (the tile's cells and one beyond either end) and W
+    if (inside) {
 #pragma unroll
-        for (int v = 0; v < NPM; ++v) t[v] = v == 5 ? 0.0 : gc[m][SL(v)];
-        adj_scatter_mhd(a, src[m], xs[m], ys[m], t);
+        for (int s = 0; s < NS; ++s) SP[s * PAD + pi] = a.Pp[G::prim(s) * a.total + g];
+        if (!MHD) SA[tid] = a.Pp[5 * a.total + g];
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) SW[q * T + tid] = inside ? a.W[q * a.total + g] : 0.0;
+    if ((valid && !inside) || ends) {
+        const int e = first ? -1 : 1;
+#pragma unroll 1
+        for (int pass = inside ? 1 : 0; pass < (ends ? 2 : 1); ++pass) {
+            const int d = pass ? e : 0;
+            const int ce = c + d;
+            double cp[NPr];
+            if (ce >= 0 && ce < nD) {
+                const long long ge = B.offset + (long long)(unsigned)((D == 0 ? ce : i) + n0 * ((D == 1 ? ce : j) + n1 * (D == 2 ? ce : k)));
+#pragma unroll
+                for (int m = 0; m < NPr; ++m) cp[m] = a.Pp[m * a.total + ge];
+            } else {
+                line_ghost_load<MHD, RARE>(a, B, D == 0 ? ce : i, D == 1 ? ce : j, D == 2 ? ce : k, cp);
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) SP[s * PAD + pi + d * step] = cp[G::prim(s)];
+            if (!MHD && pass == 0) SA[tid] = cp[5];
+        }
+    }
+    __syncthreads();
+
+    // ---------------- 2: reconstruction
+    const CellWeights w = cell_weights<RARE>(B, D, active ? c : 0);
+    const bool clean = !MHD || P.divergence_cleaning;
+    double qp[NS];
+    bool bad_p = false, bad_m = false;   // e4/onedinterp.d:44-74: the face takes the cell-centre state
+    if (active) {
+        double qm_r = 1.0, qm_u = 1.0;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const double* v = SP + pv[s] * PAD + pi;
+            double qm, rd = 0.0;
+            if (s == 8 && !clean) qp[s] = qm = v[0];
+            else cell_recon<RARE>(P, w, v[-step], v[0], v[step], qm, qp[s], rd);
+            SM[s * T + tid] = qm;
+            SR[s * T + tid] = rd;
+            if (s == 3) qm_r = qm;
+            if (s == 4) qm_u = qm;
+        }
+        bad_p = qp[4] <= 0.0 || qp[3] <= 0.0;
+        bad_m = qm_u <= 0.0 || qm_r <= 0.0;
+        if (bad_m) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s) SM[s * T + tid] = SP[pv[s] * PAD + pi];
+        }
+        if (bad_p) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s) qp[s] = SP[pv[s] * PAD + pi];
+        }
+    }
+    __syncthreads();
+
+    // ---------------- 3: flux of the plus face; qp becomes its cotangent
+    double ga = 0.0;
+    if (has_face) {
+        // cotangent of the face flux: F enters R of the right cell with +A/V and of the left with -A/V
+        double AVr = B.area[D] * B.vol_inv * a.w_scale, AVl = AVr;
+        if (RARE && B.graded) {
+            // graded: the face's area from its cells' lengths across it, each side's own volume
+            const int ic[3] = {i + (D == 0), j + (D == 1), k + (D == 2)};
+            double Lr[3], Ll[3];
+            for (int d = 0; d < 3; ++d) {
+                Lr[d] = B.glen[d][ic[d] + 2];
+                Ll[d] = B.glen[d][ic[d] - (d == D) + 2];
+            }
+            const bool threeD = P.dims == 3;
+            const double Af = threeD ? (D == 0 ? Lr[1] * Lr[2] : (D == 1 ? Lr[2] * Lr[0] : Lr[0] * Lr[1]))
+                                     : (D == 0 ? Lr[1] : Lr[0]);
+            AVr = Af * rcp(threeD ? Lr[0] * Lr[1] * Lr[2] : Lr[0] * Lr[1]) * a.w_scale;
+            AVl = Af * rcp(threeD ? Ll[0] * Ll[1] * Ll[2] : Ll[0] * Ll[1]) * a.w_scale;
+        }
+        const int nb = tid + step;   // the cell to the right
+        double gF[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            // the face's frame: momentum and B components in the order normal, tangents
+            const int qg = q >= 1 && q <= 3 ? 1 + (D + q - 1) % 3 : (MHD && q >= 5 && q <= 7 ? 5 + (D + q - 5) % 3 : q);
+            gF[q] = AVr * SW[qg * T + nb] - AVl * SW[qg * T + tid];
+        }
+        const int bface = c == -1 ? 2 * D : (c == nD - 1 ? 2 * D + 1 : -1);
+        bool simple = false;
+        if constexpr (RARE && !MHD) simple = bface >= 0 && B.bc_type[bface] == BC_SIMPLE_FLUX;
+        if constexpr (RARE && !MHD) {
+            if (simple) {
+                // OutFlowBC_SimpleFlux (boundary_flux_effect.d:504-645): the boundary face's flux is
+                // the interior cell's outflow flux, or only its pressure on a closed face
+                const int at = pi + ((bface & 1) ? 0 : step);
+                double gg[5] = {gF[MASS], 0.0, 0.0, 0.0, gF[TOTENERGY]}, cs[6], gs[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                gg[1 + ax0] = gF[1]; gg[1 + ax1] = gF[2]; gg[1 + ax2] = gF[3];
+                for (int s = 0; s < 5; ++s) cs[s] = SP[s * PAD + at];
+                cs[5] = 0.0;
+                simple_flux_vjp<D>(P, cs, (bface & 1) ? 1 : -1, gg, gs);
+                const long long gi = B.offset + (long long)(unsigned)(i + n0 * (j + n1 * k) + ((bface & 1) ? 0 : sD));
+                for (int m = 0; m < 5; ++m) atomicAdd(&a.gP[m * a.total + gi], gs[m]);
+#pragma unroll
+                for (int s = 0; s < NS; ++s) { qp[s] = 0.0; SM[s * T + nb] = 0.0; }
+                SA[T + nb] = 0.0;
+            }
+        }
+        if (!simple) {
+            double r[NS], gl[NS], gr[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) r[s] = SM[s * T + nb];
+            if constexpr (MHD) {
+                mhd_face_rev(a, qp, r, gF, gl, gr);
+            } else {
+                double gaR;
+                euler_face_rev<FLUX>(P, qp, SA[tid], r, SA[nb], gF, gl, ga, gr, gaR);
+                SA[T + nb] = gaR;
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) { qp[s] = gl[s]; SM[s * T + nb] = gr[s]; }
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) qp[s] = 0.0;
+    }
+    __syncthreads();
+
+    // ---------------- 4: reverse of the limiter; the cotangents of the cells before and after
+    // the own one go to shared memory, the own one's stays
+    double gc[NPr];
+#pragma unroll
+    for (int m = 0; m < NPr; ++m) gc[m] = 0.0;
+    if (active) {
+        if (!MHD) gc[5] = ga + (has_left ? SA[T + tid] : 0.0);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const double* v = SP + pv[s] * PAD + pi;
+            double gp = qp[s], gm = has_left ? SM[s * T + tid] : 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
+            if (bad_p) { g0 += gp; gp = 0.0; }
+            if (bad_m) { g0 += gm; gm = 0.0; }
+            if (s == 8 && !clean) g0 += gp + gm;
+            else cell_recon_rev<RARE>(P, w, v[-step], v[0], v[step], SR[s * T + tid], gp, gm, g1, g0, g2);
+            SM[s * T + tid] = g1;
+            SR[s * T + tid] = g2;
+            gc[G::prim(pv[s])] = g0;
+        }
+    }
+    __syncthreads();
+
+    // ---------------- 5: the cell's sum; ghosts pass it on by their rules
+    const bool from_left = valid && !first && c >= 0 && c - 1 <= nD;       // the cells before and after that
+    const bool from_right = valid && !last && c + 1 <= nD;                 // were active in this tile
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const int m = G::prim(pv[s]);
+        if (from_left) gc[m] += SR[s * T + tid - step];
+        if (from_right) gc[m] += SM[s * T + tid + step];
+    }
+    if (inside) {
+#pragma unroll
+        for (int m = 0; m < NPr; ++m)
+            if (!MHD || m != 5) atomicAdd(&a.gP[m * a.total + g], gc[m]);
+    }
+    // the tile's ends and the ghosts; inflow ghosts (one state a face) are summed over the tile first
+    double vin[NPr];
+    bool in = false;
+    int side = 0;
+    if ((valid && !inside && (active || from_left || from_right)) || ends) {
+        const int e = first ? -1 : 1;
+#pragma unroll 1
+        for (int pass = inside ? 1 : 0; pass < (ends ? 2 : 1); ++pass) {
+            const int ce = c + (pass ? e : 0);
+            if (pass) {
+                if (!MHD) gc[5] = 0.0;
+#pragma unroll
+                for (int s = 0; s < NS; ++s) gc[G::prim(pv[s])] = (first ? SM : SR)[s * T + tid];
+            }
+            if (ce >= 0 && ce < nD) {
+                const long long ge = B.offset + (long long)(unsigned)((D == 0 ? ce : i) + n0 * ((D == 1 ? ce : j) + n1 * (D == 2 ? ce : k)));
+#pragma unroll
+                for (int m = 0; m < NPr; ++m)
+                    if (m != 5) atomicAdd(&a.gP[m * a.total + ge], gc[m]);
+            } else {
+                side = ce < 0 ? 0 : 1;
+                if (B.bc_type[2 * D + side] == BC_INFLOW) {
+#pragma unroll
+                    for (int m = 0; m < NPr; ++m) vin[m] = (in ? vin[m] : 0.0) + gc[m];
+                    in = true;
+                } else {
+                    double t[NPr];   // (a copy, so that gc itself stays in registers)
+#pragma unroll
+                    for (int m = 0; m < NPr; ++m) t[m] = gc[m];
+                    line_ghost_scatter<MHD, RARE>(a, B, D == 0 ? ce : i, D == 1 ? ce : j, D == 2 ? ce : k, t);
+                }
+            }
+        }
+    }
+    if (B.bc_type[2 * D] == BC_INFLOW || B.bc_type[2 * D + 1] == BC_INFLOW) {
+#pragma unroll 1
+        for (int sd = 0; sd < 2; ++sd) {
+            if (!__syncthreads_or(in && side == sd)) continue;
+#pragma unroll
+            for (int m = 0; m < NPr; ++m) {
+                double v = in && side == sd ? vin[m] : 0.0;
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) SIN[warp * NPr + m] = v;
+            }
+            __syncthreads();
+            if (tid < NPr) {
+                double v = 0.0;
+                for (int wv = 0; wv < T / 32; ++wv) v += SIN[wv * NPr + tid];
+                atomicAdd(&a.gInflow[B.bc_inflow[2 * D + sd] * NPr + tid], v);
+            }
+        }
     }
 }
 
-// RARE: some exchange rotates its ghosts' vectors (the only rare rule MHD takes).
-// Each thread keeps its stencil's primitives and cotangents (nine of each per cell, 72
-// doubles) in shared memory at a stride of 73 doubles (conflict-free for 8-byte
-// accesses): 74.75 KB per CTA of 128 threads, 3 CTAs per SM at 168 registers, with the
-// carveout that gives shared memory the most room.
-constexpr int MHD_SLOT = 8 * 9 + 1;
-constexpr size_t MHD_FACE_SMEM = sizeof(double) * MHD_SLOT * 128;
-template <bool RARE>
-__global__ void __launch_bounds__(128, 3) adj_faces_mhd_kernel(AdjArgs a, unsigned nb0, unsigned nb1) {
-    extern __shared__ double smem_mhd[];
-    double* smt = smem_mhd + threadIdx.x * MHD_SLOT;
+// All tiles of the three directions in one launch: CTAs [0, nb0) take the i lines,
+// [nb0, nb0 + nb1) the j lines, the rest the k lines.
+#ifndef GDFV_ADJ_MINB
+#define GDFV_ADJ_MINB 2
+#endif
+#ifndef GDFV_ADJ_MINB_MHD
+#define GDFV_ADJ_MINB_MHD 2
+#endif
+template <bool MHD, int FLUX, bool RARE>
+__global__ void __launch_bounds__(LINE_CTA, MHD ? GDFV_ADJ_MINB_MHD : GDFV_ADJ_MINB)
+    adj_lines_kernel(const __grid_constant__ AdjArgs a, unsigned nb0, unsigned nb1) {
+    extern __shared__ double smem_lines[];
     const unsigned bid = blockIdx.x;
-    if (bid < nb0) face_mhd<0, RARE>(a, (long long)bid * 128 + threadIdx.x, smt);
-    else if (bid < nb0 + nb1) face_mhd<1, RARE>(a, (long long)(bid - nb0) * 128 + threadIdx.x, smt);
-    else face_mhd<2, RARE>(a, (long long)(bid - nb0 - nb1) * 128 + threadIdx.x, smt);
+    if (bid < nb0) line_tile<0, MHD, FLUX, RARE>(a, bid, smem_lines);
+    else if (bid < nb0 + nb1) line_tile<1, MHD, FLUX, RARE>(a, bid - nb0, smem_lines);
+    else line_tile<2, MHD, FLUX, RARE>(a, bid - nb0 - nb1, smem_lines);
 }
 
-void launch_faces_mhd(const AdjArgs& a, const unsigned* nb, cudaStream_t s) {
-    static bool attr_set[2] = {false, false};   // dynamic shared memory above 48 KB, once per instantiation
-    // (the attributes are the function's, for the process's device)
-    const int r = a.P.rotating ? 1 : 0;
-    if (!attr_set[r]) {
-        if (r) cudaFuncSetAttribute(adj_faces_mhd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MHD_FACE_SMEM);
-        else cudaFuncSetAttribute(adj_faces_mhd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MHD_FACE_SMEM);
-        if (r) cudaFuncSetAttribute(adj_faces_mhd_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        else cudaFuncSetAttribute(adj_faces_mhd_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        attr_set[r] = true;
-    }
-    const unsigned n = nb[0] + nb[1] + nb[2];
-    if (r) adj_faces_mhd_kernel<true><<<n, 128, MHD_FACE_SMEM, s>>>(a, nb[0], nb[1]);
-    else adj_faces_mhd_kernel<false><<<n, 128, MHD_FACE_SMEM, s>>>(a, nb[0], nb[1]);
+// Tiles of one direction of a block (line_tile's decomposition).
+long long line_tiles(const int* n, int D) {
+    if (D == 0) return ((long long)(n[0] + 4) * n[1] * n[2] - 1 + LINE_CTA - 2) / (LINE_CTA - 1);
+    const long long lines = (long long)n[0] * (D == 1 ? n[2] : n[1]);
+    return (lines + 31) / 32 * ((n[D] + 1 + LINE_J - 2) / (LINE_J - 1));
+}
+
+template <bool MHD, int FLUX, bool RARE>
+cudaError_t launch_lines_of(const AdjArgs& a, const unsigned* nb, cudaStream_t s) {
+    using G = LineGeo<MHD>;
+    auto* kernel = adj_lines_kernel<MHD, FLUX, RARE>;
+    // the attribute is the device's: set for every launch (a host-side table look-up)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::bytes);
+    if (e != cudaSuccess) return e;
+    kernel<<<nb[0] + nb[1] + nb[2], LINE_CTA, G::bytes, s>>>(a, nb[0], nb[1]);
+    return cudaGetLastError();
+}
+
+// The face sweep of the context's flux calculator, with the rare rules when some exchange
+// rotates, some face is an outflow boundary of its own, the limiter is lmr's or a block graded.
+cudaError_t launch_lines(const AdjArgs& a, int flux, const unsigned* nb, cudaStream_t s) {
+    const bool rare = a.P.rotating || a.P.outflow_bcs || a.P.lmr_epsilon || a.P.graded;
+    if (a.P.mhd)
+        return rare ? launch_lines_of<true, FLUX_HLLE, true>(a, nb, s) : launch_lines_of<true, FLUX_HLLE, false>(a, nb, s);
+    if (flux == FLUX_HLLC)
+        return rare ? launch_lines_of<false, FLUX_HLLC, true>(a, nb, s) : launch_lines_of<false, FLUX_HLLC, false>(a, nb, s);
+    return rare ? launch_lines_of<false, FLUX_AUSMDV, true>(a, nb, s) : launch_lines_of<false, FLUX_AUSMDV, false>(a, nb, s);
 }
 
 // MHD decode (e4/fvcell.d:586-822): the ten primitives of each cell, gP cleared.
@@ -1485,22 +1448,6 @@ using namespace gdfv;
 
 namespace {
 
-// The face kernel of the context's flux calculator (with the rare rules when some
-// exchange rotates, some face is an outflow boundary of its own or the limiter is lmr's)
-// over nb[d] CTAs of each direction.
-template <int FLUX>
-void launch_faces_flux(const AdjArgs& a, bool rare, const unsigned* nb, cudaStream_t s) {
-    const unsigned n = nb[0] + nb[1] + nb[2];
-    if (rare) adj_faces_kernel<FLUX, true><<<n, FACE_CTA, 0, s>>>(a, nb[0], nb[1]);
-    else adj_faces_kernel<FLUX, false><<<n, FACE_CTA, 0, s>>>(a, nb[0], nb[1]);
-}
-
-void launch_faces(const AdjArgs& a, int flux, const unsigned* nb, cudaStream_t s) {
-    const bool rare = a.P.rotating || a.P.outflow_bcs || a.P.lmr_epsilon || a.P.graded;
-    if (flux == FLUX_HLLC) launch_faces_flux<FLUX_HLLC>(a, rare, nb, s);
-    else launch_faces_flux<FLUX_AUSMDV>(a, rare, nb, s);
-}
-
 // The forms the VJP, step and rollout adjoints take.
 bool vjp_supported(int ctx, const AdjView& v) {
     if (!v.prepared) { adjoint_set_error(ctx, "call gdfv_prepare first"); return false; }
@@ -1522,8 +1469,8 @@ bool vjp_supported(int ctx, const AdjView& v) {
 }
 
 // Scratch layout, np = 6 primitives (Euler) or 10 (MHD), nq conserved quantities:
-// P [np][total] | gP [np][total] | b [nq][total] | face offsets [3][nblocks+1] | inflow
-// cotangents [ninflow][np].  Face offsets are uploaded once per allocation.
+// P [np][total] | gP [np][total] | b [nq][total] | tile offsets [3][nblocks+1] | inflow
+// cotangents [ninflow][np].  Tile offsets are uploaded once per allocation.
 cudaError_t vjp_setup(const AdjView& v, AdjArgs& a, std::vector<long long>& off) {
     const long long total = v.total;
     const long long np = v.mhd ? NPM : NP, nq = v.mhd ? 10 : 5;
@@ -1546,7 +1493,7 @@ cudaError_t vjp_setup(const AdjView& v, AdjArgs& a, std::vector<long long>& off)
     a.Pp = base;
     a.gP = base + np * total;
     a.bbuf = base + 2 * np * total;
-    a.face_off = reinterpret_cast<const long long*>(base + (2 * np + nq) * total);
+    a.tile_off = reinterpret_cast<const long long*>(base + (2 * np + nq) * total);
     a.gInflow = base + (2 * np + nq) * total + 3 * (v.nblocks + 1);
     a.chd_slot = a.gInflow + np * v.ninflow;   // two doubles of the tail
     a.c_h = v.c_h;
@@ -1559,13 +1506,12 @@ cudaError_t vjp_setup(const AdjView& v, AdjArgs& a, std::vector<long long>& off)
         for (int b = 0; b < v.nblocks; ++b) {
             const BlockDesc& B = v.h_blocks[b];
             // 2D blocks have no k faces (the residual sums four faces)
-            long long nf = (v.dims == 2 && d == 2) ? 0
-                                                   : (long long)(B.n[0] + (d == 0)) * (B.n[1] + (d == 1)) * (B.n[2] + (d == 2));
-            off[d * (v.nblocks + 1) + b + 1] = off[d * (v.nblocks + 1) + b] + nf;
+            const long long nt = (v.dims == 2 && d == 2) ? 0 : line_tiles(B.n, d);
+            off[d * (v.nblocks + 1) + b + 1] = off[d * (v.nblocks + 1) + b] + nt;
         }
     }
     if (!*v.scratch_ready) {
-        e = cudaMemcpy((void*)a.face_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice);
+        e = cudaMemcpy((void*)a.tile_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return e;
         *v.scratch_ready = 1;
     }
@@ -1580,9 +1526,8 @@ cudaError_t enqueue_vjp_mhd(const AdjView& v, const AdjArgs& a, const std::vecto
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     unsigned nb[3];
-    for (int d = 0; d < 3; ++d) nb[d] = (unsigned)((off[d * (v.nblocks + 1) + v.nblocks] + 127) / 128);
-    launch_faces_mhd(a, nb, v.stream);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    for (int d = 0; d < 3; ++d) nb[d] = (unsigned)off[d * (v.nblocks + 1) + v.nblocks];
+    if ((e = launch_lines(a, v.flux, nb, v.stream)) != cudaSuccess) return e;
     adj_back_mhd_kernel<<<nb_cells, nt, 0, v.stream>>>(a);
     return cudaGetLastError();
 }
@@ -1595,9 +1540,8 @@ cudaError_t enqueue_vjp(const AdjView& v, const AdjArgs& a, const std::vector<lo
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
         unsigned nb[3];
-        for (int d = 0; d < 3; ++d) nb[d] = (unsigned)((off[d * (v.nblocks + 1) + v.nblocks] + 127) / 128);
-        launch_faces(a, v.flux, nb, v.stream);
-        e = cudaGetLastError();
+        for (int d = 0; d < 3; ++d) nb[d] = (unsigned)off[d * (v.nblocks + 1) + v.nblocks];
+        e = launch_lines(a, v.flux, nb, v.stream);
     }
     if (e == cudaSuccess) {
         adj_decode_back_kernel<<<(unsigned)((total + nt - 1) / nt), nt, 0, v.stream>>>(a);
@@ -1652,10 +1596,8 @@ struct VjpChain {
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
             unsigned nb[3];
-            for (int d = 0; d < 3; ++d) nb[d] = (unsigned)((off[d * (v.nblocks + 1) + v.nblocks] + 127) / 128);
-            if (v.mhd) launch_faces_mhd(a, nb, v.stream);
-            else launch_faces(a, v.flux, nb, v.stream);
-            e = cudaGetLastError();
+            for (int d = 0; d < 3; ++d) nb[d] = (unsigned)off[d * (v.nblocks + 1) + v.nblocks];
+            e = launch_lines(a, v.flux, nb, v.stream);
         }
         back = a;
         pending = true;
