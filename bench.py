@@ -640,7 +640,7 @@ def main():
                 "d2h_bytes_per_step": (state_bytes + 64 * steps) / steps,
                 "how": "gdfv_block_set_conserved from pinned host memory, gdfv_run of all steps, "
                        "gdfv_block_get_conserved back to pinned host memory, wall clock"},
-        "gpu_launches": 4 * steps,
+        "gpu_launches": 3 * steps + 1,   # predictor, corrector, step_turn a step; step_begin
         "clocks": results["fp32"]["clocks"],
         "clocks_fp64": results["fp64"]["clocks"],
     }

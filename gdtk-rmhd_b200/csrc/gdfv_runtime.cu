@@ -30,27 +30,37 @@ struct StepParams {
 
 // e4/simcore_gasdynamic_step.d:60-160 (global dt rule) with the block rule of
 // e4/fluidblock.d:998-1095 and c_h of e4/fluidblock.d:975-995 / e4/simcore.d:1625-1648.
-// One thread; inputs are the per-block maxima of the signal frequency that the
-// previous corrector stage (or the initial scan) left behind.
-__global__ void step_begin_kernel(Control* c, const BlockDesc* blocks, unsigned long long* maxsig,
-                                  const double* lastsig, StepParams sp) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One warp, its lanes over the blocks; inputs are the per-block maxima of the signal
+// frequency that the previous corrector stage (or the initial scan) left behind.
+__device__ __forceinline__ double warp_min(double v) {
+    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ double warp_max(double v) {
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ void step_begin(Control* c, const BlockDesc* blocks, unsigned long long* maxsig, const double* lastsig,
+                           const StepParams& sp) {
+    const int lane = threadIdx.x;
     if (c->halted || c->status != ST_OK) return;
     if (c->step >= c->step_limit || (c->max_time > 0.0 && c->time >= c->max_time)) {
-        c->halted = 1;
+        __syncwarp();
+        if (lane == 0) c->halted = 1;
         return;
     }
     if (!c->retrying) {
+        double dt = c->dt_global;
         if (!sp.fixed_time_step && (c->step % sp.cfl_count) == 0) {
             const double cfl_allow = sp.n_stages == 1 ? 0.9 : (sp.n_stages == 2 ? 1.2 : 1.6);
             const double cfl_adjust = 0.5;
             const bool check_cfl = c->step > 0;
             double dt_allow_all = 1.79769313486231570e+308;
             double cfl_max_all = 0.0;
-            for (int b = 0; b < sp.nblocks; ++b) {
+            for (int b = lane; b < sp.nblocks; b += 32) {
                 double smax = __longlong_as_double((long long)maxsig[b]);
                 // max over cells of (dt*signal) and min of (cfl/signal) follow from the max signal
-                double cfl_max = c->dt_global * smax;
+                double cfl_max = dt * smax;
                 double dt_allow = sp.cfl_value / smax;
                 if (check_cfl && (cfl_max < 0.0 || cfl_max > cfl_allow)) {
                     cfl_max = cfl_adjust * cfl_allow;
@@ -59,38 +69,49 @@ __global__ void step_begin_kernel(Control* c, const BlockDesc* blocks, unsigned 
                 dt_allow_all = fmin(dt_allow_all, dt_allow);
                 cfl_max_all = fmax(cfl_max_all, cfl_max);
             }
-            c->dt_allow = dt_allow_all;
-            c->cfl_max = cfl_max_all;
-            if (c->step == 0) c->dt_allow = fmin(sp.dt_init, c->dt_allow);
-            if (c->dt_allow <= c->dt_global) {
-                c->dt_global = c->dt_allow;
+            dt_allow_all = warp_min(dt_allow_all);
+            cfl_max_all = warp_max(cfl_max_all);
+            if (c->step == 0) dt_allow_all = fmin(sp.dt_init, dt_allow_all);
+            if (dt_allow_all <= dt) {
+                dt = dt_allow_all;
             } else {
-                c->dt_global = fmin(c->dt_global * 1.5, c->dt_allow);
-                c->dt_global = fmin(c->dt_global, sp.dt_max);
+                dt = fmin(dt * 1.5, dt_allow_all);
+                dt = fmin(dt, sp.dt_max);
+            }
+            if (lane == 0) {
+                c->dt_allow = dt_allow_all;
+                c->cfl_max = cfl_max_all;
+                c->dt_global = dt;
             }
         }
         if (sp.mhd_cleaning) {
-            bool first = true;
-            for (int b = 0; b < sp.nblocks; ++b) {
+            double c_h = nan("");   // fmin takes the other operand of a NaN
+            for (int b = lane; b < sp.nblocks; b += 32) {
                 double smax = __longlong_as_double((long long)maxsig[b]);
-                double cfl_max = smax * c->dt_global;
-                double ch = cfl_max * blocks[b].L_min / c->dt_global;
-                c->c_h = first ? ch : fmin(ch, c->c_h);
-                first = false;
+                double cfl_max = smax * dt;
+                c_h = fmin(cfl_max * blocks[b].L_min / dt, c_h);
             }
+            c_h = warp_min(c_h);
+            if (lane == 0) c->c_h = c_h;
         }
-        c->t0 = c->time;
+        if (lane == 0) c->t0 = c->time;
     }
-    c->n_fail = 0;
-    c->n_invalid1 = 0;
-    c->n_invalid2 = 0;
-    c->first_bad_cell = LLONG_MAX;
-    for (int b = 0; b < sp.nblocks; ++b) maxsig[b] = 0ull;
+    if (lane == 0) {
+        c->n_fail = 0;
+        c->n_invalid1 = 0;
+        c->n_invalid2 = 0;
+        c->first_bad_cell = LLONG_MAX;
+    }
+    for (int b = lane; b < sp.nblocks; b += 32) maxsig[b] = 0ull;
+}
+
+__global__ void step_begin_kernel(Control* c, const BlockDesc* blocks, unsigned long long* maxsig,
+                                  const double* lastsig, StepParams sp) {
+    step_begin(c, blocks, maxsig, lastsig, sp);
 }
 
 // Phase 14 and the retry loop of e4/simcore_gasdynamic_step.d:1437-1560.
-__global__ void step_end_kernel(Control* c, StepParams sp) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ void step_end(Control* c, const StepParams& sp) {
     if (c->halted || c->status != ST_OK) return;
     if (c->n_fail > 0) {
         c->attempt += 1;
@@ -109,10 +130,22 @@ __global__ void step_end_kernel(Control* c, StepParams sp) {
         return;
     }
     c->time = c->t0 + c->dt_global;
+    c->dt_taken = c->dt_global;
     c->step += 1;
     c->attempt = 0;
     c->retrying = 0;
     c->steps_done += 1;
+}
+
+// Between the steps of a run: the end of one and the start of the next in one launch of one
+// warp (one thread walked the blocks before, in a launch each: with 21 blocks 86 us a step,
+// 75 with this).  A run that has reached its limit halts here, so that it needs no further
+// slot to find out.
+__global__ void step_turn_kernel(Control* c, const BlockDesc* blocks, unsigned long long* maxsig,
+                                 const double* lastsig, StepParams sp) {
+    if (threadIdx.x == 0) step_end(c, sp);
+    __syncwarp();
+    step_begin(c, blocks, maxsig, lastsig, sp);
 }
 
 struct BlockRange {
@@ -426,14 +459,19 @@ cudaError_t launch_stage(Context* c, int stage, const StageArgs& A) {
     return launch_stage_fp32(stage, c->cfg.flux, c->cfg.mhd, A, c->stream);
 }
 
+// One step of a run, which step_begin_kernel or the step before has begun.
 cudaError_t enqueue_step(Context* c) {
     StageArgs A = stage_args_run(c);
-    step_begin_kernel<<<1, 1, 0, c->stream>>>(c->d_ctl, c->d_blocks, c->d_maxsig, c->d_lastsig, c->sp);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_stage(c, 1, A);
     if (e != cudaSuccess) return e;
-    if ((e = launch_stage(c, 1, A)) != cudaSuccess) return e;
     if ((e = launch_stage(c, 2, A)) != cudaSuccess) return e;
-    step_end_kernel<<<1, 1, 0, c->stream>>>(c->d_ctl, c->sp);
+    step_turn_kernel<<<1, 32, 0, c->stream>>>(c->d_ctl, c->d_blocks, c->d_maxsig, c->d_lastsig, c->sp);
+    return cudaGetLastError();
+}
+
+// Starts a run's first step (after write_ctl).
+cudaError_t enqueue_begin(Context* c) {
+    step_begin_kernel<<<1, 32, 0, c->stream>>>(c->d_ctl, c->d_blocks, c->d_maxsig, c->d_lastsig, c->sp);
     return cudaGetLastError();
 }
 
@@ -1054,7 +1092,7 @@ __global__ void record_step_kernel(const Control* ctl, const double* U0buf, cons
     }
     const double* cur = (ctl->step & 1) ? U1buf : U0buf;
     const double* prev = (ctl->step & 1) ? U0buf : U1buf;
-    const double dt = ctl->dt_global;
+    const double dt = ctl->dt_taken;
     if (blockIdx.x == 0 && threadIdx.x == 0) *dt_out = dt;
     for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < n; x += (long long)gridDim.x * blockDim.x) {
         if (state_out) state_out[x] = cur[x];
@@ -1720,16 +1758,22 @@ int autotune(Context* c) {
     if (c->cfg.dims == 2) kcs.push_back(1);
     else {
         // chunks under 8 planes only where 8 planes a tile leave SMs without a tile, or the
-        // blocks are no deeper (their prologues cost more than the parallelism they add
-        // elsewhere: 128x128x64 FP64 510 us for both stages with 4 planes, 523 with 8;
-        // Orszag-Tang 256x256x4 FP64 276 with 4, 325 with 2)
-        double tiles8 = 0.0;
-        for (const HostBlock& hb : c->blocks)
-            tiles8 += (double)((hb.n[2] + 7) / 8) * ((hb.n[0] + 31) / 32) *
-                      ((hb.n[1] + tile_rows(c->cfg.precision, c->cfg.mhd) - 1) / tile_rows(c->cfg.precision, c->cfg.mhd));
-        const bool thin = maxk <= 8 || tiles8 < (double)c->n_sm;
-        for (int kc : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 64, 128})
-            if ((kc >= 8 || thin) && (kc <= maxk || kcs.empty())) kcs.push_back(kc);
+        // blocks are no deeper, and while the tiles fill the chip up to three times over (their
+        // prologues cost more than the parallelism they add elsewhere: 128x128x64 FP64 510 us
+        // for both stages with 4 planes, 523 with 8; Orszag-Tang 256x256x4 FP64 276 with 4, 325
+        // with 2)
+        const int TJ = tile_rows(c->cfg.precision, c->cfg.mhd);
+        auto tiles = [&](int kc) {
+            double t = 0.0;
+            for (const HostBlock& hb : c->blocks)
+                t += (double)((hb.n[2] + kc - 1) / kc) * ((hb.n[0] + 31) / 32) * ((hb.n[1] + TJ - 1) / TJ);
+            return t;
+        };
+        const bool thin = maxk <= 8 || tiles(8) < (double)c->n_sm;
+        const double most = 3.0 * c->n_sm * tile_ctas_per_sm(c->cfg.precision, c->cfg.mhd);
+        if (maxk < 8) kcs.push_back(maxk);
+        for (int kc : {128, 64, 32, 24, 16, 12, 8, 6, 4, 3, 2, 1})
+            if (kc <= maxk && (kcs.empty() || kc != kcs[0]) && (kc >= 8 || (thin && tiles(kc) <= most))) kcs.push_back(kc);
     }
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
@@ -1811,10 +1855,11 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
     c->h_ctl->max_time = max_time;
     c->h_ctl->halted = 0;
     c->h_ctl->steps_done = 0;
-    if (write_ctl(c)) return GDFV_ERR_CUDA;
     if (!c->graph) {
         if ((st = build_graph(c)) != GDFV_OK) return st;
     }
+    if (write_ctl(c)) return GDFV_ERR_CUDA;
+    CK(enqueue_begin(c));
     // Replay the captured steps in batches sized to what is left, reading the
     // control record back after each batch.  Steps past the halt are no-ops.
     const long long slot_budget = (long long)(c->cfg.max_attempts + 1) * (max_steps + 1) + 2 * c->graph_steps;
@@ -1865,10 +1910,11 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
     c->h_ctl->max_time = 0.0;
     c->h_ctl->halted = 0;
     c->h_ctl->steps_done = 0;
-    if (write_ctl(c)) return GDFV_ERR_CUDA;
     if (!c->graph) {
         if ((st = build_graph(c)) != GDFV_OK) return st;
     }
+    if (write_ctl(c)) return GDFV_ERR_CUDA;
+    CK(enqueue_begin(c));
     if (c->rec_cap < nsteps) {
         if (c->d_rec) cudaFree(c->d_rec);
         c->d_rec = nullptr;
