@@ -38,22 +38,22 @@ __device__ __forceinline__ double sgn(double x) { return x < 0.0 ? -1.0 : 1.0; }
 // Reciprocal for the adjoint arithmetic (recip, gdfv_device.cuh: within an ulp or so, no branch).
 __device__ __forceinline__ double rcp(double x) { return recip(x).r; }
 
-// Reverse of clip_to_limits(q, A, B) (src/nm/limiters.d:41-50): routes g to q, A or B.
-__device__ __forceinline__ void clip_rev(double q, double A, double B, double g, double& gq, double& gA, double& gB) {
-    bool lowerIsA = A <= B;
-    double lower = lowerIsA ? A : B;
-    bool upperIsA = A > B;
-    double upper = upperIsA ? A : B;
-    double qc = (q > lower) ? q : lower;
-    bool fromq = q > lower;
-    if (qc <= upper) {
-        if (fromq) gq += g;
-        else if (lowerIsA) gA += g;
-        else gB += g;
-    } else {
-        if (upperIsA) gA += g;
-        else gB += g;
-    }
+// clip_to_limits(q, A, B) (src/nm/limiters.d:41-50) and its reverse, which routes g to q, A or
+// B, with the order of the bounds from the sign of d = B - A (clip_by, gdfv_stage.cuh).
+__device__ __forceinline__ double clip_adj(double q, double A, double B, double d) {
+    const bool down = __double2hiint(d) < 0;
+    const double lower = down ? B : A, upper = down ? A : B;
+    const double qc = (q > lower) ? q : lower;
+    return (qc <= upper) ? qc : upper;
+}
+__device__ __forceinline__ double clip_rev(double q, double A, double B, double d, double g, double& gA, double& gB) {
+    const bool down = __double2hiint(d) < 0;
+    const double lower = down ? B : A, upper = down ? A : B;
+    const bool below = !(q > lower), above = !below && !(q <= upper), out = below || above;
+    const bool to_a = below != down;   // the lower bound is A unless down, the upper one B
+    gA += out && to_a ? g : 0.0;
+    gB += out && !to_a ? g : 0.0;
+    return out ? 0.0 : g;
 }
 
 // The l2r2 weights of one cell along a direction: both interface values of a cell come
@@ -88,16 +88,16 @@ __device__ __forceinline__ double lmr_epsilon(const NumParams& P, double toc, do
 template <bool RARE>
 __device__ __forceinline__ void cell_recon(const NumParams& P, const CellWeights& w, double q1, double q0, double q2,
                                            double& qm, double& qp, double& rd) {
-    const double dm = (q0 - q1) * w.tol, dp = (q2 - q0) * w.toc;
+    const double em = q0 - q1, ep = q2 - q0, dm = em * w.tol, dp = ep * w.toc;
     double sp = 1.0, sm = 1.0;
     rd = 0.0;
     if (P.apply_limiter) {
         const double p = dm * dp, n = p + fabs(p), d = dm * dm + dp * dp;
         if (RARE && P.lmr_epsilon) {
             int from;
-            const double ep = lmr_epsilon(P, w.toc, q0, q2, from), em = lmr_epsilon(P, w.toc, q1, q0, from);
-            sp = (n + ep) * rcp(d + ep);
-            sm = (n + em) * rcp(d + em);
+            const double lp = lmr_epsilon(P, w.toc, q0, q2, from), lm = lmr_epsilon(P, w.toc, q1, q0, from);
+            sp = (n + lp) * rcp(d + lp);
+            sm = (n + lm) * rcp(d + lm);
         } else {
             rd = rcp(d + P.eps_van_albada);
             sp = sm = (n + P.eps_van_albada) * rd;
@@ -106,8 +106,8 @@ __device__ __forceinline__ void cell_recon(const NumParams& P, const CellWeights
     qp = q0 + sp * w.a * (dp * w.twoL + dm * w.lenR0);
     qm = q0 - sm * w.a * (dp * w.lenL0 + dm * w.twoR);
     if (P.extrema_clipping) {
-        qp = clip_to_limits(qp, q0, q2);
-        qm = clip_to_limits(qm, q1, q0);
+        qp = clip_adj(qp, q0, q2, ep);
+        qm = clip_adj(qm, q1, q0, em);
     }
 }
 
@@ -116,18 +116,18 @@ __device__ __forceinline__ void cell_recon(const NumParams& P, const CellWeights
 template <bool RARE>
 __device__ __forceinline__ void cell_recon_rev(const NumParams& P, const CellWeights& w, double q1, double q0, double q2,
                                                double rd, double gp, double gm, double& g1, double& g0, double& g2) {
-    const double dm = (q0 - q1) * w.tol, dp = (q2 - q0) * w.toc;
+    const double em = q0 - q1, ep = q2 - q0, dm = em * w.tol, dp = ep * w.toc;
     const double p = dm * dp, n = p + fabs(p), d = dm * dm + dp * dp;
     const bool lmr = RARE && P.lmr_epsilon;
     double sp = 1.0, sm = 1.0, rp = rd, rm = rd;
     int fp = 0, fm = 0;
     if (P.apply_limiter) {
         if (lmr) {
-            const double ep = lmr_epsilon(P, w.toc, q0, q2, fp), em = lmr_epsilon(P, w.toc, q1, q0, fm);
-            rp = rcp(d + ep);
-            rm = rcp(d + em);
-            sp = (n + ep) * rp;
-            sm = (n + em) * rm;
+            const double lp = lmr_epsilon(P, w.toc, q0, q2, fp), lm = lmr_epsilon(P, w.toc, q1, q0, fm);
+            rp = rcp(d + lp);
+            rm = rcp(d + lm);
+            sp = (n + lp) * rp;
+            sm = (n + lm) * rm;
         } else {
             sp = sm = (n + P.eps_van_albada) * rd;
         }
@@ -136,8 +136,8 @@ __device__ __forceinline__ void cell_recon_rev(const NumParams& P, const CellWei
     g1 = g2 = 0.0;
     double gvp = 0.0, gvm = 0.0;
     if (P.extrema_clipping) {
-        clip_rev(q0 + sp * w.a * X, q0, q2, gp, gvp, g0, g2);
-        clip_rev(q0 - sm * w.a * Y, q1, q0, gm, gvm, g1, g0);
+        gvp = clip_rev(q0 + sp * w.a * X, q0, q2, ep, gp, g0, g2);
+        gvm = clip_rev(q0 - sm * w.a * Y, q1, q0, em, gm, g1, g0);
     } else {
         gvp = gp;
         gvm = gm;
@@ -155,16 +155,16 @@ __device__ __forceinline__ void cell_recon_rev(const NumParams& P, const CellWei
             gn = gnp + gnm;
             gd = gdp_ + gdm_;
             const double k = P.eps_van_albada * w.toc;   // the faces' epsilons enter n and d
-            const double ep = (gnp + gdp_) * k, em = (gnm + gdm_) * k;
-            if (fp == 1) g0 += ep * sgn(q0);
-            else if (fp == 2) g2 += ep * sgn(q2);
-            if (fm == 1) g1 += em * sgn(q1);
-            else if (fm == 2) g0 += em * sgn(q0);
+            const double kp = (gnp + gdp_) * k, km = (gnm + gdm_) * k;
+            if (fp == 1) g0 += kp * sgn(q0);
+            else if (fp == 2) g2 += kp * sgn(q2);
+            if (fm == 1) g1 += km * sgn(q1);
+            else if (fm == 2) g0 += km * sgn(q0);
         } else {
             gn = (ap * X - am * Y) * rd;
             gd = -gn * sp;
         }
-        const double gpp = gn * (1.0 + sgn(p));
+        const double gpp = p < 0.0 ? 0.0 : 2.0 * gn;   // |p| rises at 0
         gdm += gpp * dp + 2.0 * gd * dm;
         gdp += gpp * dm + 2.0 * gd * dp;
     }
