@@ -71,6 +71,11 @@ cudaError_t launch_stage_fp32(int stage, int flux, bool mhd, const StageArgs& A,
 // Primitives (rho, vel, u, a; SoA [6][total], float or double) of the state U, for the
 // kernels on decoded primitives, enqueued on stream s.
 void prims_fp32(const double* U, long long total, const NumParams& P, void* Pout, cudaStream_t s);
+// One stage (0, 1 or 2) as FP64 line sweeps (A.sweep_off set; gdfv_sweep.cuh), their tiles of
+// one direction of a block, and the FP64 primitives (6 or, MHD, 10 per cell) of the state U.
+cudaError_t launch_sweeps(int stage, int flux, bool mhd, const StageArgs& A, cudaStream_t s);
+long long sweep_tile_count(const int* n, int D, int cells);
+void prims_fp64(const double* U, long long total, const NumParams& P, bool mhd, void* Pout, cudaStream_t s);
 // Raise the dynamic shared-memory limit of every instantiation (once per device).
 cudaError_t configure_stage_fp64();
 cudaError_t configure_stage_fp32();

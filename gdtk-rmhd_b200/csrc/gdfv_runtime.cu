@@ -250,6 +250,7 @@ struct Config {
     int tile_kchunk = 0;  // 0: chosen per block
     int tile_width = 32;  // kernel on decoded primitives: tiles 32 or 16 cells wide (build_tiles)
     int persistent = 0;   // 1: stage kernels as a resident grid taking tiles from a queue
+    int line_sweeps = 2;  // FP64 stages as line sweeps: 0 never, 1 always, 2 by size
     int autotune = 0;     // time tile shapes and the launch form on the first run, keep the fastest
     int lmr_epsilon = 0;  // van_albada_variant = lmr
     double cfl_value = 0.5, dt_init = 1.0e-3, dt_max = 1.0e-3;
@@ -304,6 +305,10 @@ struct Context {
     cudaStream_t aux_stream[2] = {nullptr, nullptr};  // lowest / highest priority streams of the rollout adjoint
     void* prim[2] = {nullptr, nullptr};   // primitives of U[0], U[1] (kernels on decoded primitives)
     void* prim1 = nullptr;             // primitives of the predictor state
+    long long* d_sweep_off = nullptr;  // FP64 line sweeps: tile offsets per direction and block (null: not used)
+    double* sweep_part = nullptr;      // and the residual sums between them
+    int sweep_tiles[3] = {0, 0, 0}, sweep_cells[3] = {0, 0, 0};
+    bool sweep = false;                // the stages run as sweeps (else stage_kernel)
     bool prims_valid = false;          // prim[parity] holds the primitives of the current state
     long long last_bad_cell = -1;      // global index of the cell the last failure reported (-1: none)
     std::vector<double> h_inflow;      // supersonic-inflow states as uploaded, 9 doubles each (p, T, vel, B, psi)
@@ -320,7 +325,7 @@ struct Context {
         if (graph1) cudaGraphExecDestroy(graph1);
         for (void* p : {(void*)U[0], (void*)U[1], (void*)dU0, (void*)d_blocks, (void*)d_tiles, (void*)d_inflow,
                         (void*)d_ctl, (void*)d_maxsig, (void*)d_lastsig, (void*)d_bad, (void*)adj_scratch, (void*)jvp_scratch,
-                        (void*)norm_scratch, (void*)prim[0], (void*)prim[1], (void*)prim1, (void*)d_geom, (void*)d_rot, (void*)d_rec,
+                        (void*)norm_scratch, (void*)prim[0], (void*)prim[1], (void*)prim1, (void*)d_sweep_off, (void*)sweep_part, (void*)d_geom, (void*)d_rot, (void*)d_rec,
                         (void*)step_ctl, (void*)step_maxsig, (void*)step_lastsig, (void*)ch_maxsig,
                         (void*)ch_lastsig, (void*)ch_bad})
             if (p) cudaFree(p);
@@ -427,11 +432,30 @@ StageArgs stage_args(Context* c) {
     return A;
 }
 
+// Cells from which the FP64 stages run as line sweeps (line_sweeps 2): below it they have too
+// few lines to fill the chip.  Both stages, us, sweeps / stage_kernel at its best tiles: 48^3
+// 118 / 92, 64^3 152 / 188, 128x128x64 374 / 518; Orszag-Tang 128x128x4 133 / 120, 256x256x4
+// 240 / 277.
+constexpr long long kSweepCells = 200000;
+
+// The FP64 line sweeps in the arguments of a launch.
+void set_sweeps(const Context* c, StageArgs& A) {
+    A.sweep_off = c->d_sweep_off;
+    A.sweep_blocks = (int)c->blocks.size();
+    A.sweep_part = c->sweep_part;
+    A.prim1 = c->prim1;
+    for (int d = 0; d < 3; ++d) {
+        A.sweep_tiles[d] = c->sweep_tiles[d];
+        A.sweep_cells[d] = c->sweep_cells[d];
+    }
+}
+
 // Arguments of the context's own stepping (gdfv_run, the autotuner, gdfv_time_stages):
-// with the float Euler path, the primitive buffers of the state buffers it steps
+// with the float Euler path or the FP64 sweeps, the primitive buffers of the state buffers it steps
 // (state_parity: which of U[0], U[1] the control record's step parity 0 names).
 StageArgs stage_args_run(Context* c, int state_parity = 0) {
     StageArgs A = stage_args(c);
+    if (c->sweep) set_sweeps(c, A);
     if (c->prim[0]) {
         A.prim[0] = c->prim[state_parity];
         A.prim[1] = c->prim[state_parity ^ 1];
@@ -445,18 +469,34 @@ int read_ctl(Context* c);
 // Primitives of the current state for the kernels on decoded primitives, when the
 // state was set from outside a stage since they were last made.
 int ensure_prims(Context* c) {
-    if (!c->prim[0] || c->prims_valid) return GDFV_OK;
+    if (!c->prim[0] || c->prims_valid || (c->cfg.precision == 0 && !c->sweep)) return GDFV_OK;
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     const int parity = c->h_ctl->step & 1;
-    prims_fp32(c->U[parity], c->total, c->P, c->prim[parity], c->stream);
+    if (c->cfg.precision == 0) prims_fp64(c->U[parity], c->total, c->P, c->cfg.mhd, c->prim[parity], c->stream);
+    else prims_fp32(c->U[parity], c->total, c->P, c->prim[parity], c->stream);
     CK(cudaGetLastError());
     c->prims_valid = true;
     return GDFV_OK;
 }
 
 cudaError_t launch_stage(Context* c, int stage, const StageArgs& A) {
+    if (A.sweep_off) return launch_sweeps(stage, c->cfg.flux, c->cfg.mhd, A, c->stream);
     if (c->cfg.precision == 0) return launch_stage_fp64(stage, c->cfg.flux, c->cfg.mhd, A, c->stream);
     return launch_stage_fp32(stage, c->cfg.flux, c->cfg.mhd, A, c->stream);
+}
+
+// R(U) of a state anywhere in device memory (the sweeps decode its primitives first).
+cudaError_t launch_residual(Context* c, const double* U, double* R) {
+    StageArgs A = stage_args(c);
+    A.U_in = U;
+    A.R_out = R;
+    if (c->sweep) {
+        set_sweeps(c, A);
+        prims_fp64(U, c->total, c->P, c->cfg.mhd, c->prim1, c->stream);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return launch_stage(c, 0, A);
 }
 
 // One step of a run, which step_begin_kernel or the step before has begun.
@@ -709,6 +749,56 @@ void exchange_linear(int xm, int face, const int* n, const int* on, int* x) {
     for (int m = 0; m < 4; ++m) x[m] = (int)(unsigned)(unsigned long long)c[m];
 }
 
+// Cells per thread along direction d (1, 2) of the FP64 line sweeps: a thread walks its stretch
+// of a line cell by cell (about four cells' time more than it updates, for its start and the
+// cells at either end) and the CTAs run T / slots at a time, plus about a third of a wave for
+// the uneven end.  The stretch with the least product, among even cuts of the longest lines.
+int sweep_stretch(const Context* c, int d) {
+    const double slots = (double)c->n_sm * (c->cfg.mhd ? 2 : 4);
+    int longest = 1;
+    for (const HostBlock& hb : c->blocks) longest = std::max(longest, hb.n[d]);
+    int best = longest;
+    double least = 1e300;
+    for (int cuts = 1; cuts <= std::max(1, longest / 2); ++cuts) {
+        const int cells = (longest + cuts - 1) / cuts;
+        double tiles = 0.0;
+        for (const HostBlock& hb : c->blocks) tiles += (double)sweep_tile_count(hb.n, d, cells);
+        const double cost = (cells + 4.0) * std::max(1.0, tiles / slots + 0.35);
+        if (cost < least) { least = cost; best = cells; }
+    }
+    return best;
+}
+
+// Buffers and tile offsets of the FP64 line sweeps, when the blocks are large enough for them
+// and device memory holds them beside the state (else stage_kernel takes the stages).
+int prepare_sweeps(Context* c) {
+    if (c->cfg.line_sweeps == 0 || (c->cfg.line_sweeps == 2 && c->total < kSweepCells)) return GDFV_OK;
+    const int nb = (int)c->blocks.size();
+    std::vector<long long> off(3 * (size_t)(nb + 1), 0);
+    for (int d = 0; d < (c->cfg.dims == 3 ? 3 : 2); ++d) {
+        c->sweep_cells[d] = d == 0 ? 0 : sweep_stretch(c, d);
+        long long* o = off.data() + (size_t)d * (nb + 1);
+        for (int b = 0; b < nb; ++b) o[b + 1] = o[b] + sweep_tile_count(c->blocks[b].n, d, c->sweep_cells[d]);
+        if (o[nb] > INT_MAX) return GDFV_OK;
+        c->sweep_tiles[d] = (int)o[nb];
+    }
+    const size_t np = c->cfg.mhd ? 10 : 6, cell = sizeof(double) * (size_t)c->total;
+    const size_t obytes = sizeof(long long) * off.size();
+    c->sweep = cudaMalloc(&c->prim[0], np * cell) == cudaSuccess && cudaMalloc(&c->prim[1], np * cell) == cudaSuccess &&
+               cudaMalloc(&c->prim1, np * cell) == cudaSuccess &&
+               cudaMalloc(&c->sweep_part, (size_t)c->nq * cell) == cudaSuccess &&
+               cudaMalloc(&c->d_sweep_off, obytes) == cudaSuccess &&
+               cudaMemcpy(c->d_sweep_off, off.data(), obytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    if (!c->sweep) {
+        cudaGetLastError();
+        for (void** p : {&c->prim[0], &c->prim[1], &c->prim1, (void**)&c->sweep_part, (void**)&c->d_sweep_off}) {
+            if (*p) cudaFree(*p);
+            *p = nullptr;
+        }
+    }
+    return GDFV_OK;
+}
+
 int do_prepare(Context* c) {
     Config& g = c->cfg;
     if (c->blocks.empty()) return fail(c, GDFV_ERR_STATE, "no blocks");
@@ -922,6 +1012,10 @@ int do_prepare(Context* c) {
         CK(cudaMalloc(&c->prim[0], pbytes));
         CK(cudaMalloc(&c->prim[1], pbytes));
         CK(cudaMalloc(&c->prim1, pbytes));
+    }
+    if (g.precision == 0) {
+        const int st = prepare_sweeps(c);
+        if (st) return st;
     }
     c->prims_valid = false;
     if (!geom.empty()) {
@@ -1346,6 +1440,10 @@ int gdfv_config_set_int(int ctx, const char* key, long long value) {
         if (v != 16 && v != 32) return fail(c, GDFV_ERR_ARG, "tile_width is 16 or 32");
         g.tile_width = (int)v;
     }
+    else if (k == "line_sweeps") {
+        if (v < 0 || v > 2) return fail(c, GDFV_ERR_ARG, "line_sweeps is 0, 1 or 2");
+        g.line_sweeps = v;
+    }
     else if (k == "autotune") g.autotune = v != 0;
     else return fail(c, GDFV_ERR_ARG, "unknown integer option: " + k);
     return GDFV_OK;
@@ -1387,6 +1485,7 @@ int gdfv_config_get_double(int ctx, const char* key, double* value) {
     else if (k == "persistent") *value = g.persistent;
     else if (k == "tile_width") *value = g.tile_width;
     else if (k == "autotune") *value = g.autotune;
+    else if (k == "line_sweeps") *value = c->prepared ? (c->sweep ? 1 : 0) : g.line_sweeps;
     else if (k == "autotune_stage_ms") *value = c->tune_ms;
     else if (k == "tile_rows") *value = tile_rows(g.precision, g.mhd);
     else if (k == "tile_rows_corrector")   // the float Euler path runs both stages on the first table
@@ -1782,46 +1881,57 @@ int autotune(Context* c) {
     int best_kc = c->cfg.tile_kchunk, best_p = c->cfg.persistent, best_w = c->cfg.tile_width;
     // tile widths of the kernel on decoded primitives
     std::vector<int> widths = {c->cfg.tile_width};
-    if (c->prim[0]) widths = {32, 16};
+    if (c->prim[0] && c->cfg.precision == 1) widths = {32, 16};
     std::vector<TileDesc> tiles;
     cudaError_t e = cudaSuccess;
     const int reps = 3;
+    // one trial: the stages `reps` times after a warm-up, milliseconds for both
+    auto trial = [&](int pers) {
+        StageArgs A = stage_args_run(c, parity);
+        A.Ubuf[0] = c->U[parity];
+        A.Ubuf[1] = c->U[parity ^ 1];
+        A.ctl = c->step_ctl;
+        A.max_signal = c->step_maxsig;
+        A.last_signal = c->step_lastsig;
+        A.persistent = pers;
+        step_dt_begin_kernel<<<1, 256, 0, c->stream>>>(c->step_ctl, c->step_maxsig, (int)c->blocks.size(), 0.0, c_h);
+        e = cudaGetLastError();
+        for (int r = -1; r < reps && e == cudaSuccess; ++r) {
+            if (r == 0) e = cudaEventRecord(e0, c->stream);
+            if (e == cudaSuccess) e = launch_stage(c, 1, A);
+            if (e == cudaSuccess) e = launch_stage(c, 2, A);
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+        float ms = 0.0f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        return (double)ms / reps;
+    };
+    const double sweep_ms = c->sweep ? trial(0) : 1e30;   // the FP64 line sweeps, against stage_kernel below
+    const bool sweeps = c->sweep;
+    c->sweep = false;
     for (int tw : widths)
     for (int kc : kcs) {
         c->cfg.tile_width = tw;
         int n1 = 0, n2 = 0, n3 = 0, n4 = 0;
         build_tiles(c, kc, tiles, n1, n2, n3, n4);
         int st = upload_tiles(c, tiles, n1, n2, n3, n4);
-        if (st) { cudaEventDestroy(e0); cudaEventDestroy(e1); return st; }
+        if (st) { cudaEventDestroy(e0); cudaEventDestroy(e1); c->sweep = sweeps; return st; }
         for (int pers = 1; pers >= 0 && e == cudaSuccess; --pers) {
-            StageArgs A = stage_args_run(c, parity);
-            A.Ubuf[0] = c->U[parity];
-            A.Ubuf[1] = c->U[parity ^ 1];
-            A.ctl = c->step_ctl;
-            A.max_signal = c->step_maxsig;
-            A.last_signal = c->step_lastsig;
-            A.persistent = pers;
-            step_dt_begin_kernel<<<1, 256, 0, c->stream>>>(c->step_ctl, c->step_maxsig, (int)c->blocks.size(), 0.0, c_h);
-            e = cudaGetLastError();
-            for (int r = -1; r < reps && e == cudaSuccess; ++r) {
-                if (r == 0) e = cudaEventRecord(e0, c->stream);
-                if (e == cudaSuccess) e = launch_stage(c, 1, A);
-                if (e == cudaSuccess) e = launch_stage(c, 2, A);
-            }
-            if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
-            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-            float ms = 0.0f;
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-            if (e == cudaSuccess && ms / reps < best) { best = ms / reps; best_kc = kc; best_p = pers; best_w = tw; }
+            const double ms = trial(pers);
+            if (e == cudaSuccess && ms < best) { best = ms; best_kc = kc; best_p = pers; best_w = tw; }
         }
         if (e != cudaSuccess) break;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    c->sweep = sweeps;
     if (e != cudaSuccess) return cuda_fail(c, e, "autotune");
     c->cfg.tile_kchunk = best_kc;
     c->cfg.persistent = best_p;
     c->cfg.tile_width = best_w;
+    c->sweep = sweeps && (sweep_ms < best || c->cfg.line_sweeps == 1);
+    if (c->sweep) best = sweep_ms;
     int n1 = 0, n2 = 0, n3 = 0, n4 = 0;
     build_tiles(c, best_kc, tiles, n1, n2, n3, n4);
     int st = upload_tiles(c, tiles, n1, n2, n3, n4);
@@ -2022,10 +2132,7 @@ int gdfv_residual(int ctx, const double* U_dev, double* R_dev) {
     int st = check_ready(c, -1);
     if (st) return st;
     if (!U_dev || !R_dev) return fail(c, GDFV_ERR_ARG, "null pointer");
-    StageArgs A = stage_args(c);
-    A.U_in = U_dev;
-    A.R_out = R_dev;
-    CK(launch_stage(c, 0, A));
+    CK(launch_residual(c, U_dev, R_dev));
     CK(cudaStreamSynchronize(c->stream));
     return GDFV_OK;
 }
@@ -2059,18 +2166,13 @@ int gdfv_residual_jvp(int ctx, const double* U_dev, const double* v_dev, const d
         sigma = sum / ((double)n * vnorm);
     }
     if (sigma_used) *sigma_used = sigma;
-    StageArgs A = stage_args(c);
     if (!R0_dev) {
-        A.U_in = U_dev;
-        A.R_out = R0;
-        CK(launch_stage(c, 0, A));
+        CK(launch_residual(c, U_dev, R0));
         R0_dev = R0;
     }
     jvp_axpy_kernel<<<nb, 256, 0, c->stream>>>(U_dev, v_dev, sigma, n, Up);
     CK(cudaGetLastError());
-    A.U_in = Up;
-    A.R_out = R1;
-    CK(launch_stage(c, 0, A));
+    CK(launch_residual(c, Up, R1));
     jvp_diff_kernel<<<nb, 256, 0, c->stream>>>(R1, R0_dev, sigma, n, Jv_dev);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));

@@ -61,6 +61,12 @@ struct StageArgs {
     int n_prim_wide, n_prim_narrow;
     // rotations of exchange faces with an Rmatrix (9 doubles each, row major)
     const double* rot;
+    // FP64 line sweeps (gdfv_sweep.cuh), on the FP64 primitives in prim and prim1 (stage 0: of
+    // U_in, in prim1): prefix counts of the tiles of each direction over the blocks
+    // ([3][blocks + 1]; null: stage_kernel), their totals, cells per tile (j, k) and the residual sums
+    const long long* sweep_off;
+    int sweep_blocks, sweep_tiles[3], sweep_cells[3];
+    double* sweep_part;
 };
 
 // Compile-time geometry of the tile and of the shared-memory layout.
@@ -390,6 +396,20 @@ __device__ __forceinline__ void gather(const R* base, int stride, int idx, R* q)
 // the reference's comparisons; the float path uses min/max (the same value for
 // every non-NaN input up to the sign of a zero result).
 __device__ __forceinline__ double clip_fast(double q, double A, double B) { return clip_to_limits(q, A, B); }
+// The same with the order of A and B from the sign of the difference d = B - A that the
+// reconstruction forms anyway, read from its high word: two FP64 comparisons fewer (A = B
+// gives d = +0, and a NaN difference is the positive one, which leaves clip_to_limits' choice).
+template <class R>
+__device__ __forceinline__ R clip_by(R q, R A, R B, R d) {
+    if constexpr (sizeof(R) == 8) {
+        const bool down = __double2hiint(d) < 0;
+        const double lower = down ? B : A, upper = down ? A : B;
+        const double qc = (q > lower) ? q : lower;
+        return (qc <= upper) ? qc : upper;
+    } else {
+        return clip_fast(q, A, B);
+    }
+}
 __device__ __forceinline__ float clip_fast(float q, float A, float B) {
     return fminf(fmaxf(q, fminf(A, B)), fmaxf(A, B));
 }
@@ -417,8 +437,9 @@ __device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, co
 #pragma unroll
     for (int s = 0; s < NRS; ++s) {
         if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
-        R dm = (q0[s] - qm1[s]) * t;
-        R dp = (qp1[s] - q0[s]) * t;
+        const R em1 = q0[s] - qm1[s], ep1 = qp1[s] - q0[s];
+        R dm = em1 * t;
+        R dp = ep1 * t;
         R sl = R(1.0), slm = R(1.0);
         if (lim) {
             if (OPT == 0 && P.lmr_epsilon) {
@@ -438,8 +459,8 @@ __device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, co
         R vp = q0[s] + sl * aL0 * (dp * w3 + dm * len);
         R vm = q0[s] - slm * aR0 * (dp * len + dm * w3);
         if (clip) {
-            vp = clip_fast(vp, q0[s], qp1[s]);
-            vm = clip_fast(vm, qm1[s], q0[s]);
+            vp = clip_by(vp, q0[s], qp1[s], ep1);
+            vm = clip_by(vm, qm1[s], q0[s], em1);
         }
         qp[s] = vp;
         qm[s] = vm;
@@ -522,15 +543,16 @@ __device__ __forceinline__ void recon_cell_graded_of(const double* g, const NumP
 #pragma unroll
     for (int s = 0; s < NRS; ++s) {
         if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
-        R dm = (q0[s] - qm1[s]) * tol;
-        R dp = (qp1[s] - q0[s]) * toc;
+        const R em1 = q0[s] - qm1[s], ep1 = qp1[s] - q0[s];
+        R dm = em1 * tol;
+        R dp = ep1 * toc;
         R sl = R(1.0);
         if (P.apply_limiter) sl = limiter<R, FD>(dm, dp, eps);
         R vp = q0[s] + sl * a * (dp * twoL + dm * lenR0);
         R vm = q0[s] - sl * a * (dp * lenL0 + dm * twoR);
         if (P.extrema_clipping) {
-            vp = clip_fast(vp, q0[s], qp1[s]);
-            vm = clip_fast(vm, qm1[s], q0[s]);
+            vp = clip_by(vp, q0[s], qp1[s], ep1);
+            vm = clip_by(vm, qm1[s], q0[s], em1);
         }
         qp[s] = vp;
         qm[s] = vm;
@@ -731,10 +753,13 @@ __device__ __forceinline__ void face_flux(const NumParams& P, R c_h, const R* qL
         // 1e-30 .. 1e30) it runs with the compiler's division, out of line
         HiRange h;
         h.take(L.rho); h.take(Rr.rho); h.take(L.p); h.take(Rr.p); h.take(L.a); h.take(Rr.a);
+        // (ausmdv divides by none of the velocities but a supersonic one, |v| > a)
+        if (FLUX != FLUX_AUSMDV) {
 #pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            h.take_below(L.v[m]); h.take_below(Rr.v[m]);
-            if (MHD) { h.take_below(L.B[m]); h.take_below(Rr.B[m]); }
+            for (int m = 0; m < 3; ++m) {
+                h.take_below(L.v[m]); h.take_below(Rr.v[m]);
+                if (MHD) { h.take_below(L.B[m]); h.take_below(Rr.B[m]); }
+            }
         }
         if (h.in_range()) {
             flux_of<R, FLUX, true>(P, L, Rr, F);

@@ -28,7 +28,7 @@ _INT_KEYS = ("interpolation_order", "dimensions", "MHD", "divergence_cleaning", 
              "extrema_clipping", "apply_entropy_fix", "interpolate_in_local_frame", "stringent_cfl",
              "cfl_count", "max_attempts_for_step", "max_invalid_cells", "fixed_time_step",
              "n_ghost_cell_layers", "glm_reference_indexing", "tile_kchunk", "persistent", "tile_width",
-             "autotune")
+             "line_sweeps", "autotune")
 _DBL_KEYS = ("cfl_value", "dt_init", "dt_max", "epsilon_van_albada", "divB_damping_length",
              "flowstate_limits_max_velocity", "flowstate_limits_max_temp", "flowstate_limits_min_temp")
 
@@ -62,6 +62,7 @@ class Config:
         self.tile_kchunk = 0          # planes per tile (0: up to 32, chosen from the block sizes)
         self.persistent = False       # True: stage kernels as a resident grid over the tile queue
         self.tile_width = 32          # float Euler kernel: tiles 32 or 16 cells wide
+        self.line_sweeps = 2          # FP64 stages as line sweeps: 0 never, 1 always, 2 by size
         self.autotune = False         # time tile shapes and launch forms on the first run
         self.cfl_value = 0.5
         self.dt_init = 1.0e-3

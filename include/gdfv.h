@@ -60,10 +60,14 @@ int gdfv_context_free(int ctx);
  * stage is one resident grid taking the tiles of all blocks from a queue; default 0:
  * one CTA per tile), tile_width (float-flux Euler defaults: 32, the default, tiles 32
  * cells wide, one row per warp; 16: tiles 16 wide with two rows per warp, which leave
- * fewer lanes idle on blocks whose width is not a multiple of 32),
- * autotune (1: the first gdfv_run times the tile k-chunks, both launch forms and both
- * tile widths, and keeps the fastest).  gdfv_config_get_double also reads
- * tile_kchunk, persistent, tile_width, autotune and autotune_stage_ms (stage 1 + stage 2 time of the tuned choice), and after
+ * fewer lanes idle on blocks whose width is not a multiple of 32), line_sweeps (FP64:
+ * 1: each stage as one launch per grid direction on decoded primitives, 0: as one fused
+ * launch, 2, the default: by the number of cells; they hold 184 bytes (MHD: 320) a cell
+ * more, and are left out when the device has no room for them),
+ * autotune (1: the first gdfv_run times the tile k-chunks, both launch forms, both
+ * tile widths and the line sweeps, and keeps the fastest).  gdfv_config_get_double also reads
+ * tile_kchunk, persistent, tile_width, line_sweeps (after gdfv_prepare: whether the sweeps
+ * run), autotune and autotune_stage_ms (stage 1 + stage 2 time of the tuned choice), and after
  * gdfv_prepare tile_rows and tile_rows_corrector (rows per column tile of the stages
  * and of the corrector, which may take taller or shorter tiles of its own). */
 int gdfv_config_set_str(int ctx, const char* key, const char* value);
