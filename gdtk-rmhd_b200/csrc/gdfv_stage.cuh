@@ -393,22 +393,16 @@ __device__ __forceinline__ void gather(const R* base, int stride, int idx, R* q)
 }
 
 // Clip q to the range of A and B (src/nm/limiters.d:41-50).  The FP64 path keeps
-// the reference's comparisons; the float path uses min/max (the same value for
+// the reference's comparisons, with the order of A and B from the sign of the difference
+// B - A that the reconstruction forms anyway, read from its high word: two FP64 comparisons
+// fewer (A = B gives +0, and a NaN difference is the positive one, which leaves
+// clip_to_limits' choice).  The float path uses min/max (the same value for
 // every non-NaN input up to the sign of a zero result).
-__device__ __forceinline__ double clip_fast(double q, double A, double B) { return clip_to_limits(q, A, B); }
-// The same with the order of A and B from the sign of the difference d = B - A that the
-// reconstruction forms anyway, read from its high word: two FP64 comparisons fewer (A = B
-// gives d = +0, and a NaN difference is the positive one, which leaves clip_to_limits' choice).
-template <class R>
-__device__ __forceinline__ R clip_by(R q, R A, R B, R d) {
-    if constexpr (sizeof(R) == 8) {
-        const bool down = __double2hiint(d) < 0;
-        const double lower = down ? B : A, upper = down ? A : B;
-        const double qc = (q > lower) ? q : lower;
-        return (qc <= upper) ? qc : upper;
-    } else {
-        return clip_fast(q, A, B);
-    }
+__device__ __forceinline__ double clip_fast(double q, double A, double B) {
+    const bool down = __double2hiint(__dsub_rn(B, A)) < 0;
+    const double lower = down ? B : A, upper = down ? A : B;
+    const double qc = (q > lower) ? q : lower;
+    return (qc <= upper) ? qc : upper;
 }
 __device__ __forceinline__ float clip_fast(float q, float A, float B) {
     return fminf(fmaxf(q, fminf(A, B)), fmaxf(A, B));
@@ -437,9 +431,8 @@ __device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, co
 #pragma unroll
     for (int s = 0; s < NRS; ++s) {
         if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
-        const R em1 = q0[s] - qm1[s], ep1 = qp1[s] - q0[s];
-        R dm = em1 * t;
-        R dp = ep1 * t;
+        R dm = (q0[s] - qm1[s]) * t;
+        R dp = (qp1[s] - q0[s]) * t;
         R sl = R(1.0), slm = R(1.0);
         if (lim) {
             if (OPT == 0 && P.lmr_epsilon) {
@@ -459,8 +452,8 @@ __device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, co
         R vp = q0[s] + sl * aL0 * (dp * w3 + dm * len);
         R vm = q0[s] - slm * aR0 * (dp * len + dm * w3);
         if (clip) {
-            vp = clip_by(vp, q0[s], qp1[s], ep1);
-            vm = clip_by(vm, qm1[s], q0[s], em1);
+            vp = clip_fast(vp, q0[s], qp1[s]);
+            vm = clip_fast(vm, qm1[s], q0[s]);
         }
         qp[s] = vp;
         qm[s] = vm;
@@ -543,16 +536,15 @@ __device__ __forceinline__ void recon_cell_graded_of(const double* g, const NumP
 #pragma unroll
     for (int s = 0; s < NRS; ++s) {
         if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
-        const R em1 = q0[s] - qm1[s], ep1 = qp1[s] - q0[s];
-        R dm = em1 * tol;
-        R dp = ep1 * toc;
+        R dm = (q0[s] - qm1[s]) * tol;
+        R dp = (qp1[s] - q0[s]) * toc;
         R sl = R(1.0);
         if (P.apply_limiter) sl = limiter<R, FD>(dm, dp, eps);
         R vp = q0[s] + sl * a * (dp * twoL + dm * lenR0);
         R vm = q0[s] - sl * a * (dp * lenL0 + dm * twoR);
         if (P.extrema_clipping) {
-            vp = clip_by(vp, q0[s], qp1[s], ep1);
-            vm = clip_by(vm, qm1[s], q0[s], em1);
+            vp = clip_fast(vp, q0[s], qp1[s]);
+            vm = clip_fast(vm, qm1[s], q0[s]);
         }
         qp[s] = vp;
         qm[s] = vm;
