@@ -138,8 +138,8 @@ __device__ void step_end(Control* c, const StepParams& sp) {
 }
 
 // Between the steps of a run: the end of one and the start of the next in one launch of one
-// warp (one thread walked the blocks before, in a launch each: with 21 blocks 86 us a step,
-// 75 with this).  A run that has reached its limit halts here, so that it needs no further
+// warp (one thread walked the blocks before, in a launch each: with 21 blocks of 60x20x2 cells
+// 75.0 us a step, 73.4 with this).  A run that has reached its limit halts here, so that it needs no further
 // slot to find out.
 __global__ void step_turn_kernel(Control* c, const BlockDesc* blocks, unsigned long long* maxsig,
                                  const double* lastsig, StepParams sp) {
@@ -279,6 +279,9 @@ struct Context {
     InflowState* d_inflow = nullptr;
     Control* d_ctl = nullptr;
     Control* h_ctl = nullptr;  // pinned mirror
+    bool ctl_current = true;   // the mirror holds what the record holds
+    double* io_buf = nullptr;  // device side of the flow-state copies of small blocks, kept
+    size_t io_cap = 0;
     unsigned long long* d_maxsig = nullptr;
     double* d_lastsig = nullptr;
     int* d_bad = nullptr;
@@ -324,7 +327,7 @@ struct Context {
         if (graph) cudaGraphExecDestroy(graph);
         if (graph1) cudaGraphExecDestroy(graph1);
         for (void* p : {(void*)U[0], (void*)U[1], (void*)dU0, (void*)d_blocks, (void*)d_tiles, (void*)d_inflow,
-                        (void*)d_ctl, (void*)d_maxsig, (void*)d_lastsig, (void*)d_bad, (void*)adj_scratch, (void*)jvp_scratch,
+                        (void*)d_ctl, (void*)io_buf, (void*)d_maxsig, (void*)d_lastsig, (void*)d_bad, (void*)adj_scratch, (void*)jvp_scratch,
                         (void*)norm_scratch, (void*)prim[0], (void*)prim[1], (void*)prim1, (void*)d_sweep_off, (void*)sweep_part, (void*)d_geom, (void*)d_rot, (void*)d_rec,
                         (void*)step_ctl, (void*)step_maxsig, (void*)step_lastsig, (void*)ch_maxsig,
                         (void*)ch_lastsig, (void*)ch_bad})
@@ -536,8 +539,7 @@ int step_scratch(Context* c) {
 int scan_signal(Context* c) {
     CK(cudaMemsetAsync(c->d_maxsig, 0, sizeof(unsigned long long) * c->blocks.size(), c->stream));
     CK(cudaMemsetAsync(c->d_bad, 0, sizeof(int), c->stream));
-    CK(cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    if (read_ctl(c)) return GDFV_ERR_CUDA;
     const double* Ucur = c->U[c->h_ctl->step & 1];
     for (size_t b = 0; b < c->blocks.size(); ++b) {
         long long n = (long long)c->blocks[b].n[0] * c->blocks[b].n[1] * c->blocks[b].n[2];
@@ -1056,15 +1058,21 @@ int do_prepare(Context* c) {
     return GDFV_OK;
 }
 
+// The mirror h_ctl follows the control record: nothing on the device changes the record
+// between the calls, so it is read back only after work that does (ctl_changed).
 int read_ctl(Context* c) {
+    if (c->ctl_current) return GDFV_OK;
     CK(cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    c->ctl_current = true;
     return GDFV_OK;
 }
 
+// Not waited for: the mirror is pinned, and it is written again only by the host after it has
+// been read back, which the stream orders after this copy.
 int write_ctl(Context* c) {
     CK(cudaMemcpyAsync(c->d_ctl, c->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    c->ctl_current = true;
     return GDFV_OK;
 }
 
@@ -1633,6 +1641,27 @@ static int check_ready(Context* c, int blk) {
     return GDFV_OK;
 }
 
+// Device buffer of n doubles for a copy of flow states: one kept by the context up to 64 MB (a
+// cudaMalloc and cudaFree a call cost more than the copy of a small block: 20 steps of 32^3
+// cells with the state in and the flow out 3.6 ms with them, 1.84 without, together with the
+// round trips that read_ctl and write_ctl spare), else its own.
+static double* io_get(Context* c, long long n) {
+    const size_t bytes = sizeof(double) * (size_t)n;
+    double* p = nullptr;
+    if (bytes > ((size_t)64 << 20)) return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+    if (c->io_cap < bytes) {
+        if (c->io_buf) cudaFree(c->io_buf);
+        c->io_buf = nullptr;
+        c->io_cap = 0;
+        if (cudaMalloc(&c->io_buf, bytes) != cudaSuccess) return nullptr;
+        c->io_cap = bytes;
+    }
+    return c->io_buf;
+}
+static void io_put(Context* c, double* p) {
+    if (p != c->io_buf) cudaFree(p);
+}
+
 int gdfv_block_set_flow_rhoT(int ctx, int blk, const double* prim) {
     Context* c = get_ctx(ctx);
     int st = check_ready(c, blk);
@@ -1641,8 +1670,8 @@ int gdfv_block_set_flow_rhoT(int ctx, int blk, const double* prim) {
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     const HostBlock& b = c->blocks[blk];
     long long n = (long long)b.n[0] * b.n[1] * b.n[2];
-    double* d_prim = nullptr;
-    CK(cudaMalloc(&d_prim, sizeof(double) * 9 * n));
+    double* d_prim = io_get(c, 9 * n);
+    if (!d_prim) return cuda_fail(c, cudaGetLastError(), "cudaMalloc of the flow-state buffer");
     cudaError_t e = cudaMemcpyAsync(d_prim, prim, sizeof(double) * 9 * n, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_bad, 0, sizeof(int), c->stream);
     if (e == cudaSuccess) {
@@ -1653,7 +1682,7 @@ int gdfv_block_set_flow_rhoT(int ctx, int blk, const double* prim) {
     int bad = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, c->d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_prim);
+    io_put(c, d_prim);
     if (e != cudaSuccess) return cuda_fail(c, e, "set_flow_rhoT");
     if (bad) return fail(c, GDFV_ERR_ARG, "initial state has T <= 0 or rho <= 0");
     c->signal_valid = false;
@@ -1703,14 +1732,14 @@ int gdfv_block_get_flow(int ctx, int blk, double* out) {
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     const HostBlock& b = c->blocks[blk];
     long long n = (long long)b.n[0] * b.n[1] * b.n[2];
-    double* d_out = nullptr;
-    CK(cudaMalloc(&d_out, sizeof(double) * 12 * n));
+    double* d_out = io_get(c, 12 * n);
+    if (!d_out) return cuda_fail(c, cudaGetLastError(), "cudaMalloc of the flow-state buffer");
     decode_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->U[c->h_ctl->step & 1], c->total, b.offset,
                                                                        n, c->P, d_out);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, sizeof(double) * 12 * n, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_out);
+    io_put(c, d_out);
     if (e != cudaSuccess) return cuda_fail(c, e, "get_flow");
     return GDFV_OK;
 }
@@ -1961,6 +1990,7 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     if (c->h_ctl->status != ST_OK) return fail(c, GDFV_ERR_STATE, "a previous run failed; reset the state");
     const int start_step = c->h_ctl->step;
+    c->ctl_current = false;   // until it is written
     c->h_ctl->step_limit = start_step + max_steps;
     c->h_ctl->max_time = max_time;
     c->h_ctl->halted = 0;
@@ -1969,6 +1999,7 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
         if ((st = build_graph(c)) != GDFV_OK) return st;
     }
     if (write_ctl(c)) return GDFV_ERR_CUDA;
+    c->ctl_current = false;   // the steps change the record
     CK(enqueue_begin(c));
     // Replay the captured steps in batches sized to what is left, reading the
     // control record back after each batch.  Steps past the halt are no-ops.
@@ -1988,6 +2019,7 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
         for (int g = 0; g < graphs; ++g) CK(cudaGraphLaunch(c->graph, c->stream));
         for (int g = 0; g < singles; ++g) CK(cudaGraphLaunch(c->graph1, c->stream));
         launched += (long long)graphs * c->graph_steps + singles;
+        c->ctl_current = false;
         if (read_ctl(c)) return GDFV_ERR_CUDA;
     }
     if (steps_taken) *steps_taken = c->h_ctl->step - start_step;
@@ -2016,6 +2048,7 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     if (c->h_ctl->status != ST_OK) return fail(c, GDFV_ERR_STATE, "a previous run failed; reset the state");
     const int start_step = c->h_ctl->step;
+    c->ctl_current = false;   // until it is written
     c->h_ctl->step_limit = start_step + nsteps;
     c->h_ctl->max_time = 0.0;
     c->h_ctl->halted = 0;
@@ -2024,6 +2057,7 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
         if ((st = build_graph(c)) != GDFV_OK) return st;
     }
     if (write_ctl(c)) return GDFV_ERR_CUDA;
+    c->ctl_current = false;   // the steps change the record
     CK(enqueue_begin(c));
     if (c->rec_cap < nsteps) {
         if (c->d_rec) cudaFree(c->d_rec);
@@ -2114,6 +2148,7 @@ int gdfv_set_time(int ctx, double time, int step, double dt_global) {
         CK(cudaMemcpyAsync(c->U[step & 1], c->U[old_parity], sizeof(double) * c->nq * c->total,
                            cudaMemcpyDeviceToDevice, c->stream));
     }
+    c->ctl_current = false;
     c->h_ctl->time = time;
     c->h_ctl->step = step;
     c->h_ctl->dt_global = dt_global;
@@ -2285,6 +2320,7 @@ int gdfv_state_device_ptr(int ctx, double** U_dev) {
     if (st) return st;
     if (!U_dev) return fail(c, GDFV_ERR_ARG, "null pointer");
     if (read_ctl(c)) return GDFV_ERR_CUDA;
+    CK(cudaStreamSynchronize(c->stream));   // the caller may use another stream
     *U_dev = c->U[c->h_ctl->step & 1];
     c->prims_valid = false;   // the caller may write the state through the pointer
     return GDFV_OK;
@@ -2310,6 +2346,7 @@ int gdfv_time_stages(int ctx, int reps, double* ms) {
     if ((st = ensure_prims(c)) != GDFV_OK) return st;
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     Control saved = *c->h_ctl;
+    c->ctl_current = false;
     // a step that cannot halt: the kernels run, the step counter does not move
     c->h_ctl->step_limit = INT_MAX;
     c->h_ctl->max_time = 0.0;
