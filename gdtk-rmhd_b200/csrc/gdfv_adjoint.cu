@@ -39,7 +39,7 @@ __device__ __forceinline__ double sgn(double x) { return x < 0.0 ? -1.0 : 1.0; }
 __device__ __forceinline__ double rcp(double x) { return recip(x).r; }
 
 // clip_to_limits(q, A, B) (src/nm/limiters.d:41-50) and its reverse, which routes g to q, A or
-// B, with the order of the bounds from the sign of d = B - A (clip_by, gdfv_stage.cuh).
+// B, with the order of the bounds from the sign of d = B - A (clip_fast, gdfv_stage.cuh).
 __device__ __forceinline__ double clip_adj(double q, double A, double B, double d) {
     const bool down = __double2hiint(d) < 0;
     const double lower = down ? B : A, upper = down ? A : B;
@@ -708,7 +708,7 @@ struct Src {
 
 // RARE: some exchange rotates its ghosts' vectors, some face is an outflow boundary
 // with a ghost or flux rule of its own, the limiter is lmr's, or some block is graded
-// (the face kernels without it carry none of that code)
+// (the kernels without it carry none of that code)
 template <bool RARE>
 __device__ Src adj_resolve(const AdjArgs& a, const BlockDesc& B, int i, int j, int k) {
     StageArgs A{};
@@ -895,25 +895,35 @@ __device__ void adj_scatter_mhd(const AdjArgs& a, const Src& s, double x, double
 //   4  per cell: reverse of the limiter: cotangents of the cells before, at and after it
 //   5  per cell: their sum, added to gP (atomically: the three directions and the tiles'
 //      ends meet there)
-// Along i a tile is 256 consecutive slots of the block's lines laid end to end, each with
+// Along i a tile is 256 (MHD 192) consecutive slots of the block's lines laid end to end, each with
 // its two ghosts on either side; along j and k it is 32 lines (lanes, i fastest, so global
-// accesses are coalesced) by 8 cells.  Neighbouring tiles share their end cells: each adds
-// the part of the faces it owns (255 slots, or 7 cells, of faces).
-constexpr int LINE_CTA = 256;
-constexpr int LINE_J = 8;      // cells along j or k per tile
+// accesses are coalesced) by 8 (MHD 6) cells.  Neighbouring tiles share their end cells: each adds
+// the part of the faces it owns (all but the last slot's, or the last cell's).
+#ifndef GDFV_ADJ_J
+#define GDFV_ADJ_J 8
+#endif
+// MHD: 6 layers, 2 CTAs of 192 threads at 168 registers (0.5 KB of spills): 269 us a product
+// on Orszag-Tang 256x256x4 and 249 us at 64^3, against 298 / 263 with 8 layers at 128
+// registers (1.4 KB), 292 / 253 with 4 layers at 3 CTAs and 342 / 262 with 12 at one.  Euler: 8
+// layers, 2 CTAs at 128 registers 456 us at 128x128x64; 6 or 5 layers at 96 registers 461 / 446
+#ifndef GDFV_ADJ_J_MHD
+#define GDFV_ADJ_J_MHD 6
+#endif
 template <bool MHD>
 struct LineGeo {
+    static constexpr int J = MHD ? GDFV_ADJ_J_MHD : GDFV_ADJ_J;   // cells along j or k per tile
+    static constexpr int CTA = 32 * J;
     static constexpr int NPr = MHD ? NPM : NP;   // primitives of a cell
     static constexpr int NS = MHD ? 9 : 5;       // reconstructed scalars
     static constexpr int NQ = MHD ? 10 : 5;
-    static constexpr int PAD = (LINE_J + 2) * 32;                  // cells with one halo layer on either side
+    static constexpr int PAD = (J + 2) * 32;                  // cells with one halo layer on either side
     static constexpr int O_P = 0;                                  // [NS][PAD] reconstructed primitives
-    static constexpr int O_W = O_P + NS * PAD;                     // [NQ][256] W (zero outside the block)
-    static constexpr int O_M = O_W + NQ * LINE_CTA;                // [NS][256] minus-face state, then its cotangent, then g1
-    static constexpr int O_R = O_M + NS * LINE_CTA;                // [NS][256] limiter reciprocal, then g2
-    static constexpr int O_A = O_R + NS * LINE_CTA;                // Euler: [256] sound speed, [256] its cotangent from the left face
-    static constexpr int O_IN = O_A + (MHD ? 0 : 2 * LINE_CTA);    // [8][NPr] inflow sums of the warps
-    static constexpr int O_END = O_IN + 8 * NPr;
+    static constexpr int O_W = O_P + NS * PAD;                     // [NQ][CTA] W (zero outside the block)
+    static constexpr int O_M = O_W + NQ * CTA;                // [NS][CTA] minus-face state, then its cotangent, then g1
+    static constexpr int O_R = O_M + NS * CTA;                // [NS][CTA] limiter reciprocal, then g2
+    static constexpr int O_A = O_R + NS * CTA;                // Euler: [CTA] sound speed, [CTA] its cotangent from the left face
+    static constexpr int O_IN = O_A + (MHD ? 0 : 2 * CTA);    // [J][NPr] inflow sums of the warps
+    static constexpr int O_END = O_IN + J * NPr;
     static constexpr size_t bytes = sizeof(double) * (size_t)O_END;
     // place of primitive v among the reconstructed ones (MHD never reconstructs the sound speed)
     static __host__ __device__ constexpr int slot(int v) { return MHD && v > 5 ? v - 1 : v; }
@@ -1001,7 +1011,7 @@ __device__ __forceinline__ void mhd_face_rev(const AdjArgs& a, const double* l, 
 template <int D, bool MHD, int FLUX, bool RARE>
 __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, double* sm) {
     using G = LineGeo<MHD>;
-    constexpr int NS = G::NS, NQ = G::NQ, NPr = G::NPr, T = LINE_CTA, PAD = G::PAD;
+    constexpr int NS = G::NS, NQ = G::NQ, NPr = G::NPr, T = G::CTA, PAD = G::PAD, LINE_J = G::J;
     constexpr int ax0 = D, ax1 = (D + 1) % 3, ax2 = (D + 2) % 3;
     constexpr int step = D == 0 ? 1 : 32;   // to the next cell along D, in shared memory
     double* SP = sm + G::O_P;
@@ -1281,7 +1291,7 @@ __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, doubl
 #define GDFV_ADJ_MINB_MHD 2
 #endif
 template <bool MHD, int FLUX, bool RARE>
-__global__ void __launch_bounds__(LINE_CTA, MHD ? GDFV_ADJ_MINB_MHD : GDFV_ADJ_MINB)
+__global__ void __launch_bounds__(LineGeo<MHD>::CTA, MHD ? GDFV_ADJ_MINB_MHD : GDFV_ADJ_MINB)
     adj_lines_kernel(const __grid_constant__ AdjArgs a, unsigned nb0, unsigned nb1) {
     extern __shared__ double smem_lines[];
     const unsigned bid = blockIdx.x;
@@ -1291,11 +1301,14 @@ __global__ void __launch_bounds__(LINE_CTA, MHD ? GDFV_ADJ_MINB_MHD : GDFV_ADJ_M
 }
 
 // Tiles of one direction of a block (line_tile's decomposition).
-long long line_tiles(const int* n, int D) {
-    if (D == 0) return ((long long)(n[0] + 4) * n[1] * n[2] - 1 + LINE_CTA - 2) / (LINE_CTA - 1);
+template <bool MHD>
+long long line_tiles_of(const int* n, int D) {
+    constexpr int J = LineGeo<MHD>::J, T = LineGeo<MHD>::CTA;
+    if (D == 0) return ((long long)(n[0] + 4) * n[1] * n[2] - 1 + T - 2) / (T - 1);
     const long long lines = (long long)n[0] * (D == 1 ? n[2] : n[1]);
-    return (lines + 31) / 32 * ((n[D] + 1 + LINE_J - 2) / (LINE_J - 1));
+    return (lines + 31) / 32 * ((n[D] + 1 + J - 2) / (J - 1));
 }
+long long line_tiles(bool mhd, const int* n, int D) { return mhd ? line_tiles_of<true>(n, D) : line_tiles_of<false>(n, D); }
 
 template <bool MHD, int FLUX, bool RARE>
 cudaError_t launch_lines_of(const AdjArgs& a, const unsigned* nb, cudaStream_t s) {
@@ -1304,7 +1317,7 @@ cudaError_t launch_lines_of(const AdjArgs& a, const unsigned* nb, cudaStream_t s
     // the attribute is the device's: set for every launch (a host-side table look-up)
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::bytes);
     if (e != cudaSuccess) return e;
-    kernel<<<nb[0] + nb[1] + nb[2], LINE_CTA, G::bytes, s>>>(a, nb[0], nb[1]);
+    kernel<<<nb[0] + nb[1] + nb[2], G::CTA, G::bytes, s>>>(a, nb[0], nb[1]);
     return cudaGetLastError();
 }
 
@@ -1506,7 +1519,7 @@ cudaError_t vjp_setup(const AdjView& v, AdjArgs& a, std::vector<long long>& off)
         for (int b = 0; b < v.nblocks; ++b) {
             const BlockDesc& B = v.h_blocks[b];
             // 2D blocks have no k faces (the residual sums four faces)
-            const long long nt = (v.dims == 2 && d == 2) ? 0 : line_tiles(B.n, d);
+            const long long nt = (v.dims == 2 && d == 2) ? 0 : line_tiles(v.mhd, B.n, d);
             off[d * (v.nblocks + 1) + b + 1] = off[d * (v.nblocks + 1) + b] + nt;
         }
     }
