@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -282,6 +283,7 @@ struct Context {
     bool ctl_current = true;   // the mirror holds what the record holds
     double* io_buf = nullptr;  // device side of the flow-state copies of small blocks, kept
     size_t io_cap = 0;
+    std::atomic<bool> io_busy{false};   // some call has it: another thread's call takes its own
     unsigned long long* d_maxsig = nullptr;
     double* d_lastsig = nullptr;
     int* d_bad = nullptr;
@@ -311,6 +313,7 @@ struct Context {
     long long* d_sweep_off = nullptr;  // FP64 line sweeps: tile offsets per direction and block (null: not used)
     double* sweep_part = nullptr;      // and the residual sums between them
     int sweep_tiles[3] = {0, 0, 0}, sweep_cells[3] = {0, 0, 0};
+    void* sweep_mem = nullptr;         // the allocation that holds prim, prim1, sweep_part and d_sweep_off then
     bool sweep = false;                // the stages run as sweeps (else stage_kernel)
     bool prims_valid = false;          // prim[parity] holds the primitives of the current state
     long long last_bad_cell = -1;      // global index of the cell the last failure reported (-1: none)
@@ -328,7 +331,7 @@ struct Context {
         if (graph1) cudaGraphExecDestroy(graph1);
         for (void* p : {(void*)U[0], (void*)U[1], (void*)dU0, (void*)d_blocks, (void*)d_tiles, (void*)d_inflow,
                         (void*)d_ctl, (void*)io_buf, (void*)d_maxsig, (void*)d_lastsig, (void*)d_bad, (void*)adj_scratch, (void*)jvp_scratch,
-                        (void*)norm_scratch, (void*)prim[0], (void*)prim[1], (void*)prim1, (void*)d_sweep_off, (void*)sweep_part, (void*)d_geom, (void*)d_rot, (void*)d_rec,
+                        (void*)norm_scratch, sweep_mem ? sweep_mem : prim[0], sweep_mem ? nullptr : prim[1], sweep_mem ? nullptr : prim1, (void*)d_geom, (void*)d_rot, (void*)d_rec,
                         (void*)step_ctl, (void*)step_maxsig, (void*)step_lastsig, (void*)ch_maxsig,
                         (void*)ch_lastsig, (void*)ch_bad})
             if (p) cudaFree(p);
@@ -785,19 +788,24 @@ int prepare_sweeps(Context* c) {
         c->sweep_tiles[d] = (int)o[nb];
     }
     const size_t np = c->cfg.mhd ? 10 : 6, cell = sizeof(double) * (size_t)c->total;
-    const size_t obytes = sizeof(long long) * off.size();
-    c->sweep = cudaMalloc(&c->prim[0], np * cell) == cudaSuccess && cudaMalloc(&c->prim[1], np * cell) == cudaSuccess &&
-               cudaMalloc(&c->prim1, np * cell) == cudaSuccess &&
-               cudaMalloc(&c->sweep_part, (size_t)c->nq * cell) == cudaSuccess &&
-               cudaMalloc(&c->d_sweep_off, obytes) == cudaSuccess &&
-               cudaMemcpy(c->d_sweep_off, off.data(), obytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    // one allocation, parts on 256-byte lines (five took a millisecond more)
+    const size_t sizes[5] = {np * cell, np * cell, np * cell, (size_t)c->nq * cell, sizeof(long long) * off.size()};
+    size_t at[6] = {0};
+    for (int m = 0; m < 5; ++m) at[m + 1] = at[m] + (sizes[m] + 255) / 256 * 256;
+    void* mem = nullptr;
+    c->sweep = cudaMalloc(&mem, at[5]) == cudaSuccess &&
+               cudaMemcpy((char*)mem + at[4], off.data(), sizes[4], cudaMemcpyHostToDevice) == cudaSuccess;
     if (!c->sweep) {
         cudaGetLastError();
-        for (void** p : {&c->prim[0], &c->prim[1], &c->prim1, (void**)&c->sweep_part, (void**)&c->d_sweep_off}) {
-            if (*p) cudaFree(*p);
-            *p = nullptr;
-        }
+        if (mem) cudaFree(mem);
+        return GDFV_OK;
     }
+    c->sweep_mem = mem;
+    c->prim[0] = mem;
+    c->prim[1] = (char*)mem + at[1];
+    c->prim1 = (char*)mem + at[2];
+    c->sweep_part = (double*)((char*)mem + at[3]);
+    c->d_sweep_off = (long long*)((char*)mem + at[4]);
     return GDFV_OK;
 }
 
@@ -1059,7 +1067,7 @@ int do_prepare(Context* c) {
 }
 
 // The mirror h_ctl follows the control record: nothing on the device changes the record
-// between the calls, so it is read back only after work that does (ctl_changed).
+// between the calls, so it is read back only after work that does (ctl_current is false then).
 int read_ctl(Context* c) {
     if (c->ctl_current) return GDFV_OK;
     CK(cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, c->stream));
@@ -1644,22 +1652,29 @@ static int check_ready(Context* c, int blk) {
 // Device buffer of n doubles for a copy of flow states: one kept by the context up to 64 MB (a
 // cudaMalloc and cudaFree a call cost more than the copy of a small block: 20 steps of 32^3
 // cells with the state in and the flow out 3.6 ms with them, 1.84 without, together with the
-// round trips that read_ctl and write_ctl spare), else its own.
+// round trips that read_ctl and write_ctl spare), else, or while another thread's call has that
+// one, its own.
 static double* io_get(Context* c, long long n) {
     const size_t bytes = sizeof(double) * (size_t)n;
     double* p = nullptr;
-    if (bytes > ((size_t)64 << 20)) return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+    if (bytes > ((size_t)64 << 20) || c->io_busy.exchange(true)) return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
     if (c->io_cap < bytes) {
-        if (c->io_buf) cudaFree(c->io_buf);
+        double* old = c->io_buf;
         c->io_buf = nullptr;
         c->io_cap = 0;
-        if (cudaMalloc(&c->io_buf, bytes) != cudaSuccess) return nullptr;
+        if (old) cudaFree(old);
+        if (cudaMalloc(&c->io_buf, bytes) != cudaSuccess) {
+            c->io_buf = nullptr;
+            c->io_busy = false;
+            return nullptr;
+        }
         c->io_cap = bytes;
     }
     return c->io_buf;
 }
 static void io_put(Context* c, double* p) {
-    if (p != c->io_buf) cudaFree(p);
+    if (p == c->io_buf) c->io_busy = false;
+    else cudaFree(p);
 }
 
 int gdfv_block_set_flow_rhoT(int ctx, int blk, const double* prim) {
@@ -1902,6 +1917,10 @@ int autotune(Context* c) {
         if (maxk < 8) kcs.push_back(maxk);
         for (int kc : {128, 64, 32, 24, 16, 12, 8, 6, 4, 3, 2, 1})
             if (kc <= maxk && (kcs.empty() || kc != kcs[0]) && (kc >= 8 || (thin && tiles(kc) <= most))) kcs.push_back(kc);
+        // nearest to the depth of the size rule first: a good time early cuts the others short
+        const double d0 = std::max(1, default_kchunk(c, 32, TJ, c->n_sm));
+        std::stable_sort(kcs.begin(), kcs.end(),
+                         [&](int a, int b) { return std::max(a / d0, d0 / a) < std::max(b / d0, d0 / b); });
     }
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
@@ -1913,9 +1932,10 @@ int autotune(Context* c) {
     if (c->prim[0] && c->cfg.precision == 1) widths = {32, 16};
     std::vector<TileDesc> tiles;
     cudaError_t e = cudaSuccess;
-    const int reps = 3;
-    // one trial: the stages `reps` times after a warm-up, milliseconds for both
-    auto trial = [&](int pers) {
+    // one trial: both stages once after a warm-up, and twice more unless that was over a quarter
+    // above `bound` (a repeat varies by a few per cent, the two launch forms by 10); milliseconds
+    const double far = 1.25;
+    auto trial = [&](int pers, double bound) {
         StageArgs A = stage_args_run(c, parity);
         A.Ubuf[0] = c->U[parity];
         A.Ubuf[1] = c->U[parity ^ 1];
@@ -1925,18 +1945,26 @@ int autotune(Context* c) {
         A.persistent = pers;
         step_dt_begin_kernel<<<1, 256, 0, c->stream>>>(c->step_ctl, c->step_maxsig, (int)c->blocks.size(), 0.0, c_h);
         e = cudaGetLastError();
-        for (int r = -1; r < reps && e == cudaSuccess; ++r) {
-            if (r == 0) e = cudaEventRecord(e0, c->stream);
-            if (e == cudaSuccess) e = launch_stage(c, 1, A);
-            if (e == cudaSuccess) e = launch_stage(c, 2, A);
-        }
-        if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-        float ms = 0.0f;
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-        return (double)ms / reps;
+        auto stages = [&](int n) {
+            for (int r = 0; r < n && e == cudaSuccess; ++r) {
+                e = launch_stage(c, 1, A);
+                if (e == cudaSuccess) e = launch_stage(c, 2, A);
+            }
+        };
+        auto timed = [&](int n) {
+            float ms = 0.0f;
+            if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
+            stages(n);
+            if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+            return (double)ms;
+        };
+        stages(1);
+        const double once = timed(1);
+        return once > far * bound ? once : (once + timed(2)) / 3.0;
     };
-    const double sweep_ms = c->sweep ? trial(0) : 1e30;   // the FP64 line sweeps, against stage_kernel below
+    const double sweep_ms = c->sweep ? trial(0, 1e30) : 1e30;   // the FP64 line sweeps, against stage_kernel below
     const bool sweeps = c->sweep;
     c->sweep = false;
     for (int tw : widths)
@@ -1947,8 +1975,9 @@ int autotune(Context* c) {
         int st = upload_tiles(c, tiles, n1, n2, n3, n4);
         if (st) { cudaEventDestroy(e0); cudaEventDestroy(e1); c->sweep = sweeps; return st; }
         for (int pers = 1; pers >= 0 && e == cudaSuccess; --pers) {
-            const double ms = trial(pers);
+            const double ms = trial(pers, std::min(best, sweep_ms));
             if (e == cudaSuccess && ms < best) { best = ms; best_kc = kc; best_p = pers; best_w = tw; }
+            else if (ms > far * best) break;
         }
         if (e != cudaSuccess) break;
     }
