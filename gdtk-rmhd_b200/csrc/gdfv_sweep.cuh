@@ -10,10 +10,10 @@
 // three cells, the last plus-face state and the last flux in registers, and a cell's loads are
 // under way (cp.async into the thread's own shared memory) while the cell before it is
 // computed; along i the lanes of a warp are neighbouring cells of a row and exchange states and
-// fluxes by shuffles.  About 790 to 1,100 thread instructions per cell and sweep, 58% issue
+// fluxes by shuffles.  About 830 to 1,240 thread instructions per cell and sweep, 58% issue
 // active at 16 warps, and no re-evaluation but at the ends of stretches.  It pays with memory
 // traffic -- the primitives are read in every sweep and the sums go through memory twice,
-// about 450 B per cell and stage for Euler against 120 -- which stays below the arithmetic.
+// 400 to 440 B per cell and stage for Euler against 120 -- which stays below the arithmetic.
 //
 // Measured (both stages, one B200, stage_kernel at its best tiles / sweeps): 256^3 ausmdv 6.58
 // / 4.19 ms, 128x128x64 518 / 374 us, graded hllc 121x85x61 463 / 323 us, Orszag-Tang
