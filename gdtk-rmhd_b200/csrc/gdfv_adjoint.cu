@@ -38,19 +38,21 @@ __device__ __forceinline__ double sgn(double x) { return x < 0.0 ? -1.0 : 1.0; }
 // Reciprocal for the adjoint arithmetic (recip, gdfv_device.cuh: within an ulp or so, no branch).
 __device__ __forceinline__ double rcp(double x) { return recip(x).r; }
 
-// clip_to_limits(q, A, B) (src/nm/limiters.d:41-50) and its reverse, which routes g to q, A or
-// B, with the order of the bounds from the sign of d = B - A (clip_fast, gdfv_stage.cuh).
-__device__ __forceinline__ double clip_adj(double q, double A, double B, double d) {
-    const bool down = __double2hiint(d) < 0;
+// clip_to_limits(q, A, B) (src/nm/limiters.d:41-50; clip_fast, gdfv_stage.cuh) and its reverse,
+// which routes g to q, A or B: to the lower bound, which is A when A <= B and else B, or to the
+// upper one, A when A > B and else B.  A slip wall's ghost has v = -0 beside a cell at v = +0:
+// A <= B there, whichever the side.
+__device__ __forceinline__ double clip_adj(double q, double A, double B) {
+    const bool down = A > B;
     const double lower = down ? B : A, upper = down ? A : B;
     const double qc = (q > lower) ? q : lower;
     return (qc <= upper) ? qc : upper;
 }
-__device__ __forceinline__ double clip_rev(double q, double A, double B, double d, double g, double& gA, double& gB) {
-    const bool down = __double2hiint(d) < 0;
+__device__ __forceinline__ double clip_rev(double q, double A, double B, double g, double& gA, double& gB) {
+    const bool down = A > B;
     const double lower = down ? B : A, upper = down ? A : B;
     const bool below = !(q > lower), above = !below && !(q <= upper), out = below || above;
-    const bool to_a = below != down;   // the lower bound is A unless down, the upper one B
+    const bool to_a = below ? A <= B : down;
     gA += out && to_a ? g : 0.0;
     gB += out && !to_a ? g : 0.0;
     return out ? 0.0 : g;
@@ -106,8 +108,8 @@ __device__ __forceinline__ void cell_recon(const NumParams& P, const CellWeights
     qp = q0 + sp * w.a * (dp * w.twoL + dm * w.lenR0);
     qm = q0 - sm * w.a * (dp * w.lenL0 + dm * w.twoR);
     if (P.extrema_clipping) {
-        qp = clip_adj(qp, q0, q2, ep);
-        qm = clip_adj(qm, q1, q0, em);
+        qp = clip_adj(qp, q0, q2);
+        qm = clip_adj(qm, q1, q0);
     }
 }
 
@@ -136,8 +138,8 @@ __device__ __forceinline__ void cell_recon_rev(const NumParams& P, const CellWei
     g1 = g2 = 0.0;
     double gvp = 0.0, gvm = 0.0;
     if (P.extrema_clipping) {
-        gvp = clip_rev(q0 + sp * w.a * X, q0, q2, ep, gp, g0, g2);
-        gvm = clip_rev(q0 - sm * w.a * Y, q1, q0, em, gm, g1, g0);
+        gvp = clip_rev(q0 + sp * w.a * X, q0, q2, gp, g0, g2);
+        gvm = clip_rev(q0 - sm * w.a * Y, q1, q0, gm, g1, g0);
     } else {
         gvp = gp;
         gvm = gm;

@@ -392,14 +392,13 @@ __device__ __forceinline__ void gather(const R* base, int stride, int idx, R* q)
     for (int s = 0; s < NRS; ++s) q[s] = base[prim_var<D>(s) * stride + idx];
 }
 
-// Clip q to the range of A and B (src/nm/limiters.d:41-50).  The FP64 path keeps
-// the reference's comparisons, with the order of A and B from the sign of the difference
-// B - A that the reconstruction forms anyway, read from its high word: two FP64 comparisons
-// fewer (A = B gives +0, and a NaN difference is the positive one, which leaves
-// clip_to_limits' choice).  The float path uses min/max (the same value for
-// every non-NaN input up to the sign of a zero result).
+// Clip q to the range of A and B (src/nm/limiters.d:41-50).  FP64: clip_to_limits with one
+// comparison of the bounds for its two.  They differ for a NaN bound alone, where the lower
+// one is A instead of B, and there q is NaN with it and both give B.  (The order is not read
+// from the sign bit of B - A: that is set for A = +0, B = -0 and for some NaNs.)  The float
+// path uses min/max (the same value for every non-NaN input up to the sign of a zero result).
 __device__ __forceinline__ double clip_fast(double q, double A, double B) {
-    const bool down = __double2hiint(__dsub_rn(B, A)) < 0;
+    const bool down = A > B;
     const double lower = down ? B : A, upper = down ? A : B;
     const double qc = (q > lower) ? q : lower;
     return (qc <= upper) ? qc : upper;
