@@ -139,15 +139,19 @@ __device__ void step_end(Control* c, const StepParams& sp) {
 }
 
 // Between the steps of a run: the end of one and the start of the next in one launch of one
-// warp (one thread walked the blocks before, in a launch each: with 21 blocks of 60x20x2 cells
-// 75.0 us a step, 73.4 with this).  A run that has reached its limit halts here, so that it needs no further
-// slot to find out.
+// warp, its lanes over the blocks (with 21 blocks of 60x20x2 cells 73.4 us a step, against 75.0
+// in a launch each with one thread).  A run that has reached its limit halts here, so that it
+// needs no further slot to find out.
 __global__ void step_turn_kernel(Control* c, const BlockDesc* blocks, unsigned long long* maxsig,
                                  const double* lastsig, StepParams sp) {
     if (threadIdx.x == 0) step_end(c, sp);
     __syncwarp();
     step_begin(c, blocks, maxsig, lastsig, sp);
 }
+
+// The end of a run's last slot where no slot follows that could take the next step: a step
+// once begun has spent the signal maxima and set dt and c_h.
+__global__ void step_end_kernel(Control* c, StepParams sp) { step_end(c, sp); }
 
 struct BlockRange {
     long long offset, n;
@@ -505,13 +509,15 @@ cudaError_t launch_residual(Context* c, const double* U, double* R) {
     return launch_stage(c, 0, A);
 }
 
-// One step of a run, which step_begin_kernel or the step before has begun.
-cudaError_t enqueue_step(Context* c) {
+// One step of a run, which step_begin_kernel or the step before has begun; it begins the next
+// one unless it is the last slot.
+cudaError_t enqueue_step(Context* c, bool last = false) {
     StageArgs A = stage_args_run(c);
     cudaError_t e = launch_stage(c, 1, A);
     if (e != cudaSuccess) return e;
     if ((e = launch_stage(c, 2, A)) != cudaSuccess) return e;
-    step_turn_kernel<<<1, 32, 0, c->stream>>>(c->d_ctl, c->d_blocks, c->d_maxsig, c->d_lastsig, c->sp);
+    if (last) step_end_kernel<<<1, 1, 0, c->stream>>>(c->d_ctl, c->sp);
+    else step_turn_kernel<<<1, 32, 0, c->stream>>>(c->d_ctl, c->d_blocks, c->d_maxsig, c->d_lastsig, c->sp);
     return cudaGetLastError();
 }
 
@@ -2099,9 +2105,11 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
     CK(cudaMemsetAsync(flag, 0, sizeof(int), c->stream));
     const long long n = (long long)c->nq * c->total;
     const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 8LL * 148);
-    // one step slot per step, each followed by its record: no host round trip in between
+    // one step slot per step, each followed by its record: no host round trip in between.  The
+    // last slot begins no step: after a retry the record ends a step short of its limit.
     for (int m = 0; m < nsteps; ++m) {
-        CK(cudaGraphLaunch(c->graph1, c->stream));
+        if (m < nsteps - 1) CK(cudaGraphLaunch(c->graph1, c->stream));
+        else CK(enqueue_step(c, true));
         record_step_kernel<<<grid, 256, 0, c->stream>>>(c->d_ctl, c->U[0], c->U[1], c->dU0, n, start_step + m + 1,
                                                         states_dev[m], preds_dev[m], c->d_rec + m, flag);
         CK(cudaGetLastError());
