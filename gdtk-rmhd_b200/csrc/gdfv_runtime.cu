@@ -365,6 +365,7 @@ int fail(Context* c, int code, const std::string& msg) {
 }
 
 int cuda_fail(Context* c, cudaError_t e, const char* where) {
+    cudaGetLastError();   // a later launch's check is not to find this error
     return fail(c, GDFV_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
@@ -2007,6 +2008,22 @@ int autotune(Context* c) {
 
 }  // namespace gdfv
 
+// A launch of a run failed after its first step was begun (e): the maxima of the signal are
+// spent and the record may hold the dt of a step that was not taken.  The record goes back to
+// the last completed step (before: as the run found it), and the next run scans the state for
+// its maxima.
+static int abandon_run(Context* c, const Control& before, cudaError_t e, const char* where) {
+    c->signal_valid = false;
+    c->prims_valid = false;
+    c->ctl_current = false;
+    if (read_ctl(c) == GDFV_OK) {
+        if (c->h_ctl->step == before.step) *c->h_ctl = before;
+        else if (!c->h_ctl->retrying) c->h_ctl->dt_global = c->h_ctl->dt_taken;
+        write_ctl(c);
+    }
+    return cuda_fail(c, e, where);
+}
+
 extern "C" {
 
 int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
@@ -2025,6 +2042,7 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     if (c->h_ctl->status != ST_OK) return fail(c, GDFV_ERR_STATE, "a previous run failed; reset the state");
     const int start_step = c->h_ctl->step;
+    const Control before = *c->h_ctl;
     c->ctl_current = false;   // until it is written
     c->h_ctl->step_limit = start_step + max_steps;
     c->h_ctl->max_time = max_time;
@@ -2035,12 +2053,12 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
     }
     if (write_ctl(c)) return GDFV_ERR_CUDA;
     c->ctl_current = false;   // the steps change the record
-    CK(enqueue_begin(c));
+    cudaError_t e = enqueue_begin(c);
     // Replay the captured steps in batches sized to what is left, reading the
     // control record back after each batch.  Steps past the halt are no-ops.
     const long long slot_budget = (long long)(c->cfg.max_attempts + 1) * (max_steps + 1) + 2 * c->graph_steps;
     long long launched = 0;
-    while (!c->h_ctl->halted && c->h_ctl->status == ST_OK && launched < slot_budget) {
+    while (e == cudaSuccess && !c->h_ctl->halted && c->h_ctl->status == ST_OK && launched < slot_budget) {
         long long remaining = (long long)c->h_ctl->step_limit - c->h_ctl->step;
         if (max_time > 0.0 && c->h_ctl->dt_global > 0.0) {
             double est = std::ceil((max_time - c->h_ctl->time) / c->h_ctl->dt_global) + 1.0;
@@ -2051,12 +2069,14 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
         remaining = std::max<long long>(1, remaining);
         const int graphs = (int)std::min<long long>(64, remaining / c->graph_steps);
         const int singles = graphs < 64 ? (int)(remaining % c->graph_steps) : 0;
-        for (int g = 0; g < graphs; ++g) CK(cudaGraphLaunch(c->graph, c->stream));
-        for (int g = 0; g < singles; ++g) CK(cudaGraphLaunch(c->graph1, c->stream));
+        for (int g = 0; g < graphs && e == cudaSuccess; ++g) e = cudaGraphLaunch(c->graph, c->stream);
+        for (int g = 0; g < singles && e == cudaSuccess; ++g) e = cudaGraphLaunch(c->graph1, c->stream);
+        if (e != cudaSuccess) break;
         launched += (long long)graphs * c->graph_steps + singles;
         c->ctl_current = false;
         if (read_ctl(c)) return GDFV_ERR_CUDA;
     }
+    if (e != cudaSuccess) return abandon_run(c, before, e, "launch of a step");
     if (steps_taken) *steps_taken = c->h_ctl->step - start_step;
     if (c->h_ctl->status == ST_TOO_MANY_BAD_CELLS)
         return fail(c, GDFV_ERR_BAD_CELLS, "Too many bad cells during explicit gasdynamic update." +
@@ -2083,6 +2103,16 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
     if (read_ctl(c)) return GDFV_ERR_CUDA;
     if (c->h_ctl->status != ST_OK) return fail(c, GDFV_ERR_STATE, "a previous run failed; reset the state");
     const int start_step = c->h_ctl->step;
+    if (c->rec_cap < nsteps) {
+        if (c->d_rec) cudaFree(c->d_rec);
+        c->d_rec = nullptr;
+        c->rec_cap = 0;
+        CK(cudaMalloc(&c->d_rec, sizeof(double) * ((size_t)nsteps + 1)));
+        c->rec_cap = nsteps;
+    }
+    int* flag = reinterpret_cast<int*>(c->d_rec + nsteps);
+    CK(cudaMemsetAsync(flag, 0, sizeof(int), c->stream));
+    const Control before = *c->h_ctl;
     c->ctl_current = false;   // until it is written
     c->h_ctl->step_limit = start_step + nsteps;
     c->h_ctl->max_time = 0.0;
@@ -2093,27 +2123,19 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
     }
     if (write_ctl(c)) return GDFV_ERR_CUDA;
     c->ctl_current = false;   // the steps change the record
-    CK(enqueue_begin(c));
-    if (c->rec_cap < nsteps) {
-        if (c->d_rec) cudaFree(c->d_rec);
-        c->d_rec = nullptr;
-        c->rec_cap = 0;
-        CK(cudaMalloc(&c->d_rec, sizeof(double) * ((size_t)nsteps + 1)));
-        c->rec_cap = nsteps;
-    }
-    int* flag = reinterpret_cast<int*>(c->d_rec + nsteps);
-    CK(cudaMemsetAsync(flag, 0, sizeof(int), c->stream));
+    cudaError_t e = enqueue_begin(c);
     const long long n = (long long)c->nq * c->total;
     const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 8LL * 148);
     // one step slot per step, each followed by its record: no host round trip in between.  The
     // last slot begins no step: after a retry the record ends a step short of its limit.
-    for (int m = 0; m < nsteps; ++m) {
-        if (m < nsteps - 1) CK(cudaGraphLaunch(c->graph1, c->stream));
-        else CK(enqueue_step(c, true));
+    for (int m = 0; m < nsteps && e == cudaSuccess; ++m) {
+        e = m < nsteps - 1 ? cudaGraphLaunch(c->graph1, c->stream) : enqueue_step(c, true);
+        if (e != cudaSuccess) break;
         record_step_kernel<<<grid, 256, 0, c->stream>>>(c->d_ctl, c->U[0], c->U[1], c->dU0, n, start_step + m + 1,
                                                         states_dev[m], preds_dev[m], c->d_rec + m, flag);
-        CK(cudaGetLastError());
+        e = cudaGetLastError();
     }
+    if (e != cudaSuccess) return abandon_run(c, before, e, "launch of a recorded step");
     int h_flag = 0;
     CK(cudaMemcpyAsync(&h_flag, flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(dts, c->d_rec, sizeof(double) * nsteps, cudaMemcpyDeviceToHost, c->stream));
