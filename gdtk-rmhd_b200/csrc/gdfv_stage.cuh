@@ -28,6 +28,8 @@
 //            dU1 = R(U1);   U2 = U0 + dt*(0.5*dU0 + 0.5*dU1)  -> stored
 // giving 5 passes of the state per step.
 #pragma once
+#include <type_traits>
+
 #include "gdfv_device.cuh"
 
 namespace gdfv {
@@ -386,8 +388,8 @@ __device__ __forceinline__ constexpr int prim_var(int s) {
 }
 
 // Gather the reconstructed scalars of direction D from a prim array.
-template <class R, int NRS, int D>
-__device__ __forceinline__ void gather(const R* base, int stride, int idx, R* q) {
+template <class R, int NRS, int D, class From = const R>
+__device__ __forceinline__ void gather(From* base, int stride, int idx, R* q) {
 #pragma unroll
     for (int s = 0; s < NRS; ++s) q[s] = base[prim_var<D>(s) * stride + idx];
 }
@@ -407,26 +409,37 @@ __device__ __forceinline__ float clip_fast(float q, float A, float B) {
     return fminf(fmaxf(q, fminf(A, B)), fmaxf(A, B));
 }
 
-// num / den of the limiter for an epsilon whose denominators quot() does not take.
+// num / den of the limiter for a denominator that quot() does not take.
 static __device__ __noinline__ double limiter_quotient(double num, double den) { return num / den; }
 // The limiter of a scalar (e4/onedinterp.d:367-371): (p + |p| + eps) / (dm^2 + dp^2 + eps), p = dm dp.
+// FD: top gathers the high words of the denominators.
 template <class R, bool FD>
-__device__ __forceinline__ R limiter(R dm, R dp, R eps) {
+__device__ __forceinline__ R limiter(R dm, R dp, R eps, unsigned& top) {
     const R num = dm * dp + rabs(dm * dp) + eps, den = dm * dm + dp * dp + eps;
-    if constexpr (FD) return quot(num, recip(den));
-    else if constexpr (sizeof(R) == 8) return limiter_quotient(num, den);
-    else return num / den;
+    if constexpr (FD) {
+        top = max(top, (unsigned)__double2hiint(den));
+        return quot(num, recip(den));
+    } else if constexpr (sizeof(R) == 8) {
+        return limiter_quotient(num, den);
+    } else {
+        return num / den;
+    }
 }
+// The limiters' denominators of a cell suit quot(): below 2^300 (differences of about 1e45 a
+// cell length), no infinity and no NaN.  Their lower end is epsilon (eps_in_range).
+__device__ __forceinline__ bool denominators_in_range(unsigned top) { return top < (1023u + 300u) << 20; }
 
-// The operations of interp_l2r2_scalar in the reference's order (FD: quot for the limiter).
+// The operations of interp_l2r2_scalar in the reference's order (FD: quot for the limiter; the
+// result holds if denominators_in_range of what is returned).
 template <class R, int NRS, bool MHD, int OPT, bool FD>
-__device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, const R* qm1, const R* q0, const R* qp1,
+__device__ __forceinline__ unsigned recon_cell_of(const R* w, const NumParams& P, const R* qm1, const R* q0, const R* qp1,
                                               R* qm, R* qp) {
     const R t = w[W_TOC];
     const R aL0 = w[W_AL0], aR0 = w[W_AR0], len = w[W_LENL0], w3 = w[W_TWOL];
     const bool lim = OPT == 1 ? true : (bool)P.apply_limiter;
     const bool clip = OPT == 1 ? true : (bool)P.extrema_clipping;
     const R eps = R(P.eps_van_albada);
+    unsigned top = 0u;
 #pragma unroll
     for (int s = 0; s < NRS; ++s) {
         if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
@@ -441,10 +454,10 @@ __device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, co
                 const R tiny = R(1e-12);
                 const R ep = rmax(rmax(tiny, rabs(q0[s])), rmax(tiny, rabs(qp1[s]))) * eps * t;
                 const R em = rmax(rmax(tiny, rabs(qm1[s])), rmax(tiny, rabs(q0[s]))) * eps * t;
-                sl = limiter<R, FD>(dm, dp, ep);
-                slm = limiter<R, FD>(dm, dp, em);
+                sl = limiter<R, FD>(dm, dp, ep, top);
+                slm = limiter<R, FD>(dm, dp, em, top);
             } else {
-                sl = limiter<R, FD>(dm, dp, eps);
+                sl = limiter<R, FD>(dm, dp, eps, top);
                 slm = sl;
             }
         }
@@ -457,6 +470,7 @@ __device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, co
         qp[s] = vp;
         qm[s] = vm;
     }
+    return top;
 }
 
 // One cell, one direction: both interface values of every reconstructed scalar
@@ -476,7 +490,7 @@ __device__ __forceinline__ void recon_cell_of(const R* w, const NumParams& P, co
 // 2.5e-7 * cell length, far below float rounding of the reconstructed fields.
 enum : int { WF_EPS = 0, WF_P1, WF_P2, WF_R1, WF_R2, WF_N };
 template <class R, int NRS, bool MHD, int OPT>
-__device__ __forceinline__ void recon_cell(const R* w, const R* wf, const NumParams& P, const R* qm1, const R* q0,
+__device__ __forceinline__ bool recon_cell(const R* w, const R* wf, const NumParams& P, const R* qm1, const R* q0,
                                            const R* qp1, R* qm, R* qp) {
     if constexpr (sizeof(R) == 4 && OPT == 1) {
         const R e = wf[WF_EPS], P1 = wf[WF_P1], P2 = wf[WF_P2], R1 = wf[WF_R1], R2 = wf[WF_R2];
@@ -512,33 +526,34 @@ __device__ __forceinline__ void recon_cell(const R* w, const R* wf, const NumPar
         }
     } else {
         // FP64: the scalars' limiter quotients without branches (quot), so that they run
-        // interleaved; per scalar and out of line for an epsilon out of quot's range
-        if constexpr (sizeof(R) == 8) {
-            if (P.eps_in_range) {
-                recon_cell_of<R, NRS, MHD, OPT, true>(w, P, qm1, q0, qp1, qm, qp);
-                return;
-            }
-        }
-        recon_cell_of<R, NRS, MHD, OPT, false>(w, P, qm1, q0, qp1, qm, qp);
+        // interleaved; false, with nothing of value in qm and qp, where epsilon or a
+        // denominator is out of quot's range (recon_cell_of<false> then takes the cell)
+        if constexpr (sizeof(R) == 8)
+            return P.eps_in_range &&
+                   denominators_in_range(recon_cell_of<R, NRS, MHD, OPT, true>(w, P, qm1, q0, qp1, qm, qp));
+        else
+            recon_cell_of<R, NRS, MHD, OPT, false>(w, P, qm1, q0, qp1, qm, qp);
     }
+    return true;
 }
 
 // recon_cell for a cell of a graded block: the weights g[GW_*] of the cell's position
 // along the direction (e4/onedinterp.d:338-386 with the lengths of cells c-1, c, c+1;
 // the two scaled differences are those of both faces of the cell, as on a uniform grid).
 template <class R, int NRS, bool MHD, bool FD>
-__device__ __forceinline__ void recon_cell_graded_of(const double* g, const NumParams& P, const R* qm1, const R* q0,
-                                                  const R* qp1, R* qm, R* qp) {
+__device__ __forceinline__ unsigned recon_cell_graded_of(const double* g, const NumParams& P, const R* qm1,
+                                                         const R* q0, const R* qp1, R* qm, R* qp) {
     const R tol = R(g[GW_TOL]), toc = R(g[GW_TOC]), a = R(g[GW_A]);
     const R twoL = R(g[GW_TWOL]), lenR0 = R(g[GW_LENR0]), lenL0 = R(g[GW_LENL0]), twoR = R(g[GW_TWOR]);
     const R eps = R(P.eps_van_albada);
+    unsigned top = 0u;
 #pragma unroll
     for (int s = 0; s < NRS; ++s) {
         if (MHD && s == 8 && !P.divergence_cleaning) { qm[s] = q0[s]; qp[s] = q0[s]; continue; }
         R dm = (q0[s] - qm1[s]) * tol;
         R dp = (qp1[s] - q0[s]) * toc;
         R sl = R(1.0);
-        if (P.apply_limiter) sl = limiter<R, FD>(dm, dp, eps);
+        if (P.apply_limiter) sl = limiter<R, FD>(dm, dp, eps, top);
         R vp = q0[s] + sl * a * (dp * twoL + dm * lenR0);
         R vm = q0[s] - sl * a * (dp * lenL0 + dm * twoR);
         if (P.extrema_clipping) {
@@ -548,17 +563,16 @@ __device__ __forceinline__ void recon_cell_graded_of(const double* g, const NumP
         qp[s] = vp;
         qm[s] = vm;
     }
+    return top;
 }
 template <class R, int NRS, bool MHD>
-__device__ __forceinline__ void recon_cell_graded(const double* g, const NumParams& P, const R* qm1, const R* q0,
+__device__ __forceinline__ bool recon_cell_graded(const double* g, const NumParams& P, const R* qm1, const R* q0,
                                                   const R* qp1, R* qm, R* qp) {
-    if constexpr (sizeof(R) == 8) {
-        if (P.eps_in_range) {
-            recon_cell_graded_of<R, NRS, MHD, true>(g, P, qm1, q0, qp1, qm, qp);
-            return;
-        }
-    }
+    if constexpr (sizeof(R) == 8)
+        return P.eps_in_range &&
+               denominators_in_range(recon_cell_graded_of<R, NRS, MHD, true>(g, P, qm1, q0, qp1, qm, qp));
     recon_cell_graded_of<R, NRS, MHD, false>(g, P, qm1, q0, qp1, qm, qp);
+    return true;
 }
 
 // AUSMDV (e4/fluxcalc.d:477-651) for the float-flux ideal-gas variant.  The
@@ -740,19 +754,7 @@ __device__ __forceinline__ void face_flux(const NumParams& P, R c_h, const R* qL
     Rr.a = pr[5 * stride + ir];
     R F[NQ];
     if constexpr (sizeof(R) == 8) {
-        // the flux's divisors are sums and products of these; out of range (outside about
-        // 1e-30 .. 1e30) it runs with the compiler's division, out of line
-        HiRange h;
-        h.take(L.rho); h.take(Rr.rho); h.take(L.p); h.take(Rr.p); h.take(L.a); h.take(Rr.a);
-        // (ausmdv divides by none of the velocities but a supersonic one, |v| > a)
-        if (FLUX != FLUX_AUSMDV) {
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                h.take_below(L.v[m]); h.take_below(Rr.v[m]);
-                if (MHD) { h.take_below(L.B[m]); h.take_below(Rr.B[m]); }
-            }
-        }
-        if (h.in_range()) {
+        if (flux_in_range<FLUX>(L.rho, L.p, L.a, L.v, L.B, Rr.rho, Rr.p, Rr.a, Rr.v, Rr.B)) {
             flux_of<R, FLUX, true>(P, L, Rr, F);
         } else {
             const FluxVec G = flux_out_of_range<FLUX>(P.gas, P.apply_entropy_fix, L, Rr);
@@ -977,13 +979,33 @@ __global__ void __launch_bounds__(32 * (TJ + 1), MHD ? (sizeof(R) == 4 ? GDFV_MI
 
         auto slot = [&](int kk) -> R* { return ring + (((kk % 3) + 3) % 3) * NPV * PLANE; };
         // reconstruction of the cell at position pos along direction D (graded blocks take
-        // the weights of that position; only the general kernels have graded blocks)
-        auto recon = [&](int D, int pos, const R* qm1, const R* q0, const R* qp1, R* qm, R* qp) {
-            if (OPT == 0 && B.graded)
-                recon_cell_graded<R, NRS, MHD>(B.gw[D] + (pos + 1) * GW_N, P, qm1, q0, qp1, qm, qp);
-            else
-                recon_cell<R, NRS, MHD, OPT>(w[D], wf[D], P, qm1, q0, qp1, qm, qp);
+        // the weights of that position; only the general kernels have graded blocks) from the
+        // planes b1, b0, b2 at i1, i0, i2: the cells before, at and after it
+        auto recon = [&](auto dir, int pos, const R* b1, int i1, const R* b0, int i0, const R* b2, int i2, R* qm, R* qp) {
+            constexpr int D = decltype(dir)::value;
+            R qm1[NRS], q0[NRS], qp1[NRS];
+            gather<R, NRS, D>(b1, PLANE, i1, qm1);
+            gather<R, NRS, D>(b0, PLANE, i0, q0);
+            gather<R, NRS, D>(b2, PLANE, i2, qp1);
+            if (OPT == 0 && B.graded) {
+                if (recon_cell_graded<R, NRS, MHD>(B.gw[D] + (pos + 1) * GW_N, P, qm1, q0, qp1, qm, qp)) return;
+            } else {
+                if (recon_cell<R, NRS, MHD, OPT>(w[D], wf[D], P, qm1, q0, qp1, qm, qp)) return;
+            }
+            if constexpr (sizeof(R) == 8) {
+                // read again: kept until here, the 3 NRS values would spill
+                gather<R, NRS, D, const volatile R>(b1, PLANE, i1, qm1);
+                gather<R, NRS, D, const volatile R>(b0, PLANE, i0, q0);
+                gather<R, NRS, D, const volatile R>(b2, PLANE, i2, qp1);
+                if (OPT == 0 && B.graded)
+                    recon_cell_graded_of<R, NRS, MHD, false>(B.gw[D] + (pos + 1) * GW_N, P, qm1, q0, qp1, qm, qp);
+                else
+                    recon_cell_of<R, NRS, MHD, OPT, false>(w[D], P, qm1, q0, qp1, qm, qp);
+            }
         };
+        const std::integral_constant<int, 0> dir0{};
+        const std::integral_constant<int, 1> dir1{};
+        const std::integral_constant<int, 2> dir2{};
 
         R kq_prev_p[NRS];        // k-direction q+ of the current plane (left state of its top face)
         R fB[NQ];                // flux through the bottom face of the owner's cell
@@ -1005,20 +1027,14 @@ __global__ void __launch_bounds__(32 * (TJ + 1), MHD ? (sizeof(R) == 4 ? GDFV_MI
                 load_two<STAGE, FAST, MHD, NQ, OPT == 0>(A, Uin, B, dt, damp, true, false, ci, cj, ck2, pr);
                 put_prim<R, NPV>(slot(t.k0), PLANE, pidx, pr[0]);
                 // q+ of plane k0-1 (left state of face k0-1/2); own column only
-                R qm1[NRS], q0[NRS], qp1[NRS], qm[NRS];
-                gather<R, NRS, 2>(slot(t.k0 - 2), PLANE, pidx, qm1);
-                gather<R, NRS, 2>(slot(t.k0 - 1), PLANE, pidx, q0);
-                gather<R, NRS, 2>(slot(t.k0), PLANE, pidx, qp1);
-                recon(2, t.k0 - 1, qm1, q0, qp1, qm, kq_prev_p);
+                R qm[NRS];
+                recon(dir2, t.k0 - 1, slot(t.k0 - 2), pidx, slot(t.k0 - 1), pidx, slot(t.k0), pidx, qm, kq_prev_p);
                 // plane k0+1 replaces k0-2 in the ring
                 int ck3[2] = {t.k0 + 1, 0};
                 load_two<STAGE, FAST, MHD, NQ, OPT == 0>(A, Uin, B, dt, damp, true, false, ci, cj, ck3, pr);
                 put_prim<R, NPV>(slot(t.k0 + 1), PLANE, pidx, pr[0]);
                 R qkm[NRS], qkp[NRS];
-                gather<R, NRS, 2>(slot(t.k0 - 1), PLANE, pidx, qm1);
-                gather<R, NRS, 2>(slot(t.k0), PLANE, pidx, q0);
-                gather<R, NRS, 2>(slot(t.k0 + 1), PLANE, pidx, qp1);
-                recon(2, t.k0, qm1, q0, qp1, qkm, qkp);
+                recon(dir2, t.k0, slot(t.k0 - 1), pidx, slot(t.k0), pidx, slot(t.k0 + 1), pidx, qkm, qkp);
                 face_flux<R, MHD, FLUX, 2, NPV>(P, c_hR, kq_prev_p, qkm, slot(t.k0 - 1), pidx, slot(t.k0), pidx, PLANE,
                                                 fB);
 #pragma unroll
@@ -1107,23 +1123,14 @@ __global__ void __launch_bounds__(32 * (TJ + 1), MHD ? (sizeof(R) == 4 ? GDFV_MI
 
             // ---------------- phase B: reconstruction
             R kq_m[NRS], kq_p[NRS];
-            if (active && has_k) {
-                R qm1[NRS], q0[NRS], qp1[NRS];
-                gather<R, NRS, 2>(cur, PLANE, pidx, qm1);
-                gather<R, NRS, 2>(nx1, PLANE, pidx, q0);
-                gather<R, NRS, 2>(nx2, PLANE, pidx, qp1);
-                recon(2, k + 1, qm1, q0, qp1, kq_m, kq_p);
-            }
+            if (active && has_k) recon(dir2, k + 1, cur, pidx, nx1, pidx, nx2, pidx, kq_m, kq_p);
             for (int f = f0; f < NRI + NRJ && f < fend; f += fstride) {
-                R qm1[NRS], q0[NRS], qp1[NRS], qm[NRS], qp[NRS];
+                R qm[NRS], qp[NRS];
                 if (f < NRI) {
                     const int row = f / (TI + 2), ci = f % (TI + 2) - 1;   // cells -1..TI
                     if (row >= nj_t || ci > ni_t) continue;
                     const int p = (ci + 2) + PW * (row + 2);
-                    gather<R, NRS, 0>(cur, PLANE, p - 1, qm1);
-                    gather<R, NRS, 0>(cur, PLANE, p, q0);
-                    gather<R, NRS, 0>(cur, PLANE, p + 1, qp1);
-                    recon(0, t.i0 + ci, qm1, q0, qp1, qm, qp);
+                    recon(dir0, t.i0 + ci, cur, p - 1, cur, p, cur, p + 1, qm, qp);
 #pragma unroll
                     for (int s = 0; s < NRS; ++s) { RI[s * NRI + f] = qm[s]; RI[(NRS + s) * NRI + f] = qp[s]; }
                 } else {
@@ -1131,10 +1138,7 @@ __global__ void __launch_bounds__(32 * (TJ + 1), MHD ? (sizeof(R) == 4 ? GDFV_MI
                     const int cj = g / TI - 1, col = g % TI;               // rows -1..TJ
                     if (col >= ni_t || cj > nj_t) continue;
                     const int p = (col + 2) + PW * (cj + 2);
-                    gather<R, NRS, 1>(cur, PLANE, p - PW, qm1);
-                    gather<R, NRS, 1>(cur, PLANE, p, q0);
-                    gather<R, NRS, 1>(cur, PLANE, p + PW, qp1);
-                    recon(1, t.j0 + cj, qm1, q0, qp1, qm, qp);
+                    recon(dir1, t.j0 + cj, cur, p - PW, cur, p, cur, p + PW, qm, qp);
 #pragma unroll
                     for (int s = 0; s < NRS; ++s) { RJ[s * NRJ + g] = qm[s]; RJ[(NRS + s) * NRJ + g] = qp[s]; }
                 }

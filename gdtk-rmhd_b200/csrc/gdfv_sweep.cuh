@@ -232,6 +232,19 @@ __device__ __forceinline__ void sweep_finish(const StageArgs& A, int stage, cons
     }
 }
 
+// The reconstruction of a cell (values before, at and after it) whose limiters are out of the
+// branch-free quotients' range: minus- and plus-face values.
+template <int N>
+struct Values { double q[N]; };
+template <int NRS, bool MHD, int OPT>
+__device__ __noinline__ Values<2 * NRS> recon_out_of_range(const NumParams& P, const double* w, bool graded,
+                                                           Values<NRS> q1, Values<NRS> q0, Values<NRS> q2) {
+    Values<2 * NRS> r;
+    if (OPT == 0 && graded) recon_cell_graded_of<double, NRS, MHD, false>(w, P, q1.q, q0.q, q2.q, r.q, r.q + NRS);
+    else recon_cell_of<double, NRS, MHD, OPT, false>(w, P, q1.q, q0.q, q2.q, r.q, r.q + NRS);
+    return r;
+}
+
 // D: direction; LAST: the sweep that finishes the stage (k, or j in 2D).  A.sweep_part holds the
 // residual sums between sweeps; stage 0 reads the primitives of its state from A.prim1.
 template <bool MHD, int FLUX, int OPT, int D, bool LAST>
@@ -271,10 +284,22 @@ __global__ void __launch_bounds__(SWEEP_LINES, MHD ? GDFV_MARCH_MINB_MHD : GDFV_
         gather<double, NRS, D>(lo, 1, 0, q1);
         gather<double, NRS, D>(at, 1, 0, q0);
         gather<double, NRS, D>(hi, 1, 0, q2);
-        if (OPT == 0 && B.graded)
-            recon_cell_graded<double, NRS, MHD>(B.gw[D] + (long long)(c + 1) * GW_N, P, q1, q0, q2, qm, qp);
-        else
-            recon_cell<double, NRS, MHD, OPT>(B.w[D], nullptr, P, q1, q0, q2, qm, qp);
+        bool done;
+        const double* gw = nullptr;
+        if (OPT == 0 && B.graded) {
+            gw = B.gw[D] + (long long)(c + 1) * GW_N;
+            done = recon_cell_graded<double, NRS, MHD>(gw, P, q1, q0, q2, qm, qp);
+        } else {
+            done = recon_cell<double, NRS, MHD, OPT>(B.w[D], nullptr, P, q1, q0, q2, qm, qp);
+        }
+        if (!done) {
+            Values<NRS> v1, v0, v2;
+#pragma unroll
+            for (int s = 0; s < NRS; ++s) { v1.q[s] = q1[s]; v0.q[s] = q0[s]; v2.q[s] = q2[s]; }
+            const Values<2 * NRS> r = recon_out_of_range<NRS, MHD, OPT>(P, gw ? gw : B.w[D], gw != nullptr, v1, v0, v2);
+#pragma unroll
+            for (int s = 0; s < NRS; ++s) { qm[s] = r.q[s]; qp[s] = r.q[NRS + s]; }
+        }
     };
     auto flux = [&](const BlockDesc& B, int c, const double* lo, const double* at, const double* qL,
                     const double* qR, double* F) {
