@@ -35,8 +35,25 @@ constexpr int NP = 6;  // rho, v0, v1, v2, u, a
 
 __device__ __forceinline__ double sgn(double x) { return x < 0.0 ? -1.0 : 1.0; }
 
-// Reciprocal for the adjoint arithmetic (recip, gdfv_device.cuh: within an ulp or so, no branch).
-__device__ __forceinline__ double rcp(double x) { return recip(x).r; }
+// Reciprocals and roots for the adjoint arithmetic: FD: without branches (recip, root,
+// gdfv_device.cuh), for operands known to be in their range; else, and where no range is known
+// (rcp), 0, subnormal and infinite operands give what 1 / x and sqrt(x) give.
+__device__ __noinline__ double rcp_out_of_range(double x) { return 1.0 / x; }
+template <bool FD>
+__device__ __forceinline__ double rcp_of(double x) {
+    if constexpr (FD) return recip(x).r;
+    else return rcp_out_of_range(x);
+}
+template <bool FD>
+__device__ __forceinline__ double sqrt_of(double x) {
+    if constexpr (FD) return root(x);
+    else return sqrt(x);
+}
+__device__ __forceinline__ double rcp(double x) {
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    if (h - ((1023u - 1000u) << 20) >= 2000u << 20) return rcp_out_of_range(x);
+    return recip(x).r;
+}
 
 // clip_to_limits(q, A, B) (src/nm/limiters.d:41-50; clip_fast, gdfv_stage.cuh) and its reverse,
 // which routes g to q, A or B: to the lower bound, which is A when A <= B and else B, or to the
@@ -86,10 +103,11 @@ __device__ __forceinline__ double lmr_epsilon(const NumParams& P, double toc, do
 // Both interface values of one scalar of a cell (q1, q0, q2: the cells before, at and after
 // it): qm at its minus face, qp at its plus face (e4/onedinterp.d:357-386, clipping as
 // src/nm/limiters.d:41-50).  rd: the reciprocal of the limiter's denominator, for the
-// reverse (not with lmr, whose two faces have limiters of their own).
-template <bool RARE>
+// reverse (not with lmr, whose two faces have limiters of their own).  top gathers the high words
+// of the denominators; with FD the result holds if denominators_in_range(top).
+template <bool RARE, bool FD>
 __device__ __forceinline__ void cell_recon(const NumParams& P, const CellWeights& w, double q1, double q0, double q2,
-                                           double& qm, double& qp, double& rd) {
+                                           double& qm, double& qp, double& rd, unsigned& top) {
     const double em = q0 - q1, ep = q2 - q0, dm = em * w.tol, dp = ep * w.toc;
     double sp = 1.0, sm = 1.0;
     rd = 0.0;
@@ -98,10 +116,12 @@ __device__ __forceinline__ void cell_recon(const NumParams& P, const CellWeights
         if (RARE && P.lmr_epsilon) {
             int from;
             const double lp = lmr_epsilon(P, w.toc, q0, q2, from), lm = lmr_epsilon(P, w.toc, q1, q0, from);
-            sp = (n + lp) * rcp(d + lp);
-            sm = (n + lm) * rcp(d + lm);
+            sp = (n + lp) * rcp_of<FD>(d + lp);
+            sm = (n + lm) * rcp_of<FD>(d + lm);
+            top = max(top, max((unsigned)__double2hiint(d + lp), (unsigned)__double2hiint(d + lm)));
         } else {
-            rd = rcp(d + P.eps_van_albada);
+            rd = rcp_of<FD>(d + P.eps_van_albada);
+            top = max(top, (unsigned)__double2hiint(d + P.eps_van_albada));
             sp = sm = (n + P.eps_van_albada) * rd;
         }
     }
@@ -179,19 +199,20 @@ __device__ __forceinline__ void cell_recon_rev(const NumParams& P, const CellWei
 // then its reverse.  Face-local states: r, p, u (normal), v, w (tangential), e, a.
 struct FS { double r, p, u, v, w, e, a; };
 
+template <bool FD>
 __device__ void ausmdv_vjp(const NumParams& P, const FS& L, const FS& R, const double* gF, FS& gL, FS& gR) {
     // ---- forward
-    const double irL = rcp(L.r), irR = rcp(R.r);
+    const double irL = rcp_of<FD>(L.r), irR = rcp_of<FD>(R.r);
     double pLrL = L.p * irL, pRrR = R.p * irR;
     double keL = 0.5 * (L.u * L.u + L.v * L.v + L.w * L.w);
     double keR = 0.5 * (R.u * R.u + R.v * R.v + R.w * R.w);
     double HL = L.e + pLrL + keL, HR = R.e + pRrR + keR;
     double S = pLrL + pRrR;
-    const double iS = rcp(S);
+    const double iS = rcp_of<FD>(S);
     double alphaL = 2.0 * pLrL * iS, alphaR = 2.0 * pRrR * iS;
     bool amL = L.a >= R.a;
     double am = fmax(L.a, R.a);
-    const double iam = rcp(am);
+    const double iam = rcp_of<FD>(am);
     double ML = L.u * iam, MR = R.u * iam;
     double duL = 0.5 * (L.u + fabs(L.u));
     bool subL = fabs(ML) <= 1.0;
@@ -206,7 +227,7 @@ __device__ void ausmdv_vjp(const NumParams& P, const FS& L, const FS& R, const d
     double dp0 = L.p - R.p;
     bool minL = L.p <= R.p;
     double mp = fmin(L.p, R.p);
-    const double imp = rcp(mp);
+    const double imp = rcp_of<FD>(mp);
     double dpa = 10.0 * fabs(dp0) * imp;
     bool sLin = dpa < 1.0;
     double s = 0.5 * fmin(1.0, dpa);
@@ -276,7 +297,7 @@ __device__ void ausmdv_vjp(const NumParams& P, const FS& L, const FS& R, const d
         gu_L += g_Q * 2.0 * (L.u + am) * (0.25 * iam);
         g_am += g_Q * ((L.u + am) * (0.5 * iam) - QL * iam);
     } else {
-        const double iuL = rcp(L.u);
+        const double iuL = rcp_of<FD>(L.u);
         gp_L += g_pLplus * duL * iuL;
         g_duL += g_pLplus * L.p * iuL;
         gu_L -= g_pLplus * L.p * duL * iuL * iuL;
@@ -292,7 +313,7 @@ __device__ void ausmdv_vjp(const NumParams& P, const FS& L, const FS& R, const d
         gu_R += g_Q * (-2.0 * (R.u - am) * (0.25 * iam));
         g_am += g_Q * ((R.u - am) * (0.5 * iam) - QR * iam);
     } else {
-        const double iuR = rcp(R.u);
+        const double iuR = rcp_of<FD>(R.u);
         gp_R += g_pRminus * duR * iuR;
         g_duR += g_pRminus * R.p * iuR;
         gu_R -= g_pRminus * R.p * duR * iuR * iuR;
@@ -320,30 +341,31 @@ __device__ void ausmdv_vjp(const NumParams& P, const FS& L, const FS& R, const d
 // needs, then its reverse.  The Roe-averaged ratio of specific heats is gamma itself for
 // one gas (its derivative vanishes); the wave-speed min/max and the star/side switches
 // take the branches the primal values took.
+template <bool FD>
 __device__ void hllc_vjp(const NumParams& P, const FS& L, const FS& R, const double* gF, FS& gL, FS& gR) {
     // ---- forward
     const double g = P.gas.gamma;
     const double keL = 0.5 * (L.u * L.u + L.v * L.v + L.w * L.w);
     const double keR = 0.5 * (R.u * R.u + R.v * R.v + R.w * R.w);
     const double EL = L.r * L.e + L.r * keL, ER = R.r * R.e + R.r * keR;
-    const double srL = root(L.r), srR = root(R.r);
-    const double D = srL + srR, iD = rcp(D);
+    const double srL = sqrt_of<FD>(L.r), srR = sqrt_of<FD>(R.r);
+    const double D = srL + srR, iD = rcp_of<FD>(D);
     const double uhat = (srL * L.u + srR * R.u) * iD;
     const double ghat = (srL * g + srR * g) * iD;
     const double N1 = srL * L.a * L.a + srR * R.a * R.a;
-    const double sD = root(D), isD = rcp(sD);
+    const double sD = sqrt_of<FD>(D), isD = rcp_of<FD>(sD);
     const double T = D * isD;
     const double du = R.u - L.u;
     const double c2 = 0.5 * (ghat - 1.0);
     const double ahat2 = N1 * iD + c2 * T * du * du;
-    const double ahat = root(ahat2);
+    const double ahat = sqrt_of<FD>(ahat2);
     const bool SLfromL = fmin(L.u - L.a, uhat - ahat) == L.u - L.a;
     const double SL = fmin(L.u - L.a, uhat - ahat);
     const bool SRfromR = fmax(R.u + R.a, uhat + ahat) == R.u + R.a;
     const double SR = fmax(R.u + R.a, uhat + ahat);
     const double num = R.p - L.p + L.r * L.u * (SL - L.u) - R.r * R.u * (SR - R.u);
     const double den = L.r * (SL - L.u) - R.r * (SR - R.u);
-    const double iden = rcp(den);
+    const double iden = rcp_of<FD>(den);
     const double Ss = num * iden;
     const bool left = Ss > 0.0;
     const FS& X = left ? L : R;
@@ -370,7 +392,7 @@ __device__ void hllc_vjp(const NumParams& P, const FS& L, const FS& R, const dou
         gS += gF[ZMOM] * (coeff - X.r) * X.w; gc += gF[ZMOM] * S * X.w; gr -= gF[ZMOM] * S * X.w;
         gw += gF[ZMOM] * S * (coeff - X.r);
         // U* = coeff (E/r + (S* - u) (S* + p/(r (S - u))))
-        const double ir = rcp(X.r), Su = S - X.u, iSu = rcp(Su);
+        const double ir = rcp_of<FD>(X.r), Su = S - X.u, iSu = rcp_of<FD>(Su);
         const double Z = X.p * ir * iSu;
         const double Bq = Ss - X.u, Cq = Ss + Z;
         const double Xs = E * ir + Bq * Cq;
@@ -415,7 +437,7 @@ __device__ void hllc_vjp(const NumParams& P, const FS& L, const FS& R, const dou
     if (SLfromL) { gu_L += gSL; ga_L -= gSL; } else { guhat += gSL; gahat -= gSL; }
     if (SRfromR) { gu_R += gSR; ga_R += gSR; } else { guhat += gSR; gahat += gSR; }
     // ahat2 = N1 / D + c2 T du^2, T = D / sqrt(D); ahat = sqrt(ahat2)
-    const double gah2 = gahat * 0.5 * rcp(ahat);
+    const double gah2 = gahat * 0.5 * rcp_of<FD>(ahat);
     const double gN1 = gah2 * iD;
     double gD = -gah2 * N1 * iD * iD;
     double gsrL = gN1 * L.a * L.a, gsrR = gN1 * R.a * R.a;
@@ -428,7 +450,7 @@ __device__ void hllc_vjp(const NumParams& P, const FS& L, const FS& R, const dou
     gsrR += guhat * R.u * iD; gu_R += guhat * srR * iD;
     gD -= guhat * uhat * iD;
     gsrL += gD; gsrR += gD;
-    gr_L += gsrL * 0.5 * rcp(srL); gr_R += gsrR * 0.5 * rcp(srR);
+    gr_L += gsrL * 0.5 * rcp_of<FD>(srL); gr_R += gsrR * 0.5 * rcp_of<FD>(srR);
     gL = FS{gr_L, gp_L, gu_L, gv_L, gw_L, ge_L, ga_L};
     gR = FS{gr_R, gp_R, gu_R, gv_R, gw_R, ge_R, ga_R};
 }
@@ -488,29 +510,31 @@ struct FastSpeed {   // cf = sqrt(0.5 (alf + sqrt(alf^2 - 4 a2 ca2))) with its p
     double a2, ca2, alf, als, cf, ir;   // ir = 1 / rho
     bool live;        // SAFESQRT took the root
 };
+template <bool FD>
 __device__ __forceinline__ FastSpeed fast_speed(double gam, double p, double rho, double Bx, double By, double Bz) {
     FastSpeed f;
     const double BB = Bx * Bx + By * By + Bz * Bz;
-    f.ir = rcp(rho);
+    f.ir = rcp_of<FD>(rho);
     f.a2 = gam * p * f.ir;
     f.ca2 = Bx * Bx * f.ir;
     f.alf = f.a2 + BB * f.ir;
     const double X = f.alf * f.alf - 4.0 * f.a2 * f.ca2;
     f.live = fabs(X) > 1.0e-14;
-    f.als = f.live ? root(X) : 0.0;
-    f.cf = root(0.5 * (f.alf + f.als));
+    f.als = f.live ? sqrt_of<FD>(X) : 0.0;
+    f.cf = sqrt_of<FD>(0.5 * (f.alf + f.als));
     return f;
 }
 // reverse of fast_speed: gcf into the cotangents of p, rho and B (added)
+template <bool FD>
 __device__ __forceinline__ void fast_speed_rev(const FastSpeed& f, double gam, double Bx, double By, double Bz,
                                                double gcf, double& gp, double& grho, double& gBx, double& gBy,
                                                double& gBz) {
-    const double gcf2 = gcf * 0.5 * rcp(f.cf);
+    const double gcf2 = gcf * 0.5 * rcp_of<FD>(f.cf);
     double galf = 0.5 * gcf2;
     const double gals = galf;
     double ga2 = 0.0, gca2 = 0.0;
     if (f.live) {
-        const double gX = gals * 0.5 * rcp(f.als);
+        const double gX = gals * 0.5 * rcp_of<FD>(f.als);
         galf += gX * 2.0 * f.alf;
         ga2 += -4.0 * f.ca2 * gX;
         gca2 += -4.0 * f.a2 * gX;
@@ -580,14 +604,15 @@ __device__ __forceinline__ void mhd_side_flux_rev(const FSm& S, const double* gf
 
 // gF: cotangent of the face-local flux in the order MASS, XMOM, YMOM, ZMOM, TOTENERGY, XB,
 // YB, ZB; gL, gR receive the cotangents of the two states (added).
+template <bool FD>
 __device__ void hlle_mhd_vjp(const NumParams& P, const FSm& L, const FSm& R, const double* gF, FSm& gL, FSm& gR) {
     // ---- forward
-    const double gam = (P.gas.Cv + P.gas.R) * P.gas.Cvinv, igm1 = rcp(gam - 1.0);
+    const double gam = (P.gas.Cv + P.gas.R) * P.gas.Cvinv, igm1 = rcp_of<FD>(gam - 1.0);
     const double rho = 0.5 * (L.r + R.r), p = 0.5 * (L.p + R.p), u = 0.5 * (L.u + R.u);
     const double Bx = 0.5 * (L.Bx + R.Bx), By = 0.5 * (L.By + R.By), Bz = 0.5 * (L.Bz + R.Bz);
-    const FastSpeed fm = fast_speed(gam, p, rho, Bx, By, Bz);
-    const FastSpeed fL = fast_speed(gam, L.p, L.r, L.Bx, L.By, L.Bz);
-    const FastSpeed fR = fast_speed(gam, R.p, R.r, R.Bx, R.By, R.Bz);
+    const FastSpeed fm = fast_speed<FD>(gam, p, rho, Bx, By, Bz);
+    const FastSpeed fL = fast_speed<FD>(gam, L.p, L.r, L.Bx, L.By, L.Bz);
+    const FastSpeed fR = fast_speed<FD>(gam, R.p, R.r, R.Bx, R.By, R.Bz);
     const double wp = u + fm.cf, wm = u - fm.cf, wmL = L.u - fL.cf, wpR = R.u + fR.cf;
     const bool blL = wmL <= wm, brR = wpR >= wp;
     const double bl = blL ? wmL : wm, br = brR ? wpR : wp;
@@ -603,7 +628,7 @@ __device__ void hlle_mhd_vjp(const NumParams& P, const FSm& L, const FSm& R, con
     const double d[8] = {R.r - L.r, R.r * R.u - L.r * L.u, R.r * R.v - L.r * L.v, R.r * R.w - L.r * L.w,
                          (R.p - L.p) * igm1 + 0.5 * (R.r * uuR + BBR) - 0.5 * (L.r * uuL + BBL),
                          R.Bx - L.Bx, R.By - L.By, R.Bz - L.Bz};
-    const double iden = rcp(brp - blm), fac1 = brp * blm;
+    const double iden = rcp_of<FD>(brp - blm), fac1 = brp * blm;
     // ---- reverse
     double gbrp = 0.0, gblm = 0.0, gfac1 = 0.0, giden = 0.0;
     double gfLF[8], gfRF[8], gd[8];
@@ -630,9 +655,9 @@ __device__ void hlle_mhd_vjp(const NumParams& P, const FSm& L, const FSm& R, con
     // wp = u + cf, wm = u - cf of the averages
     const double gu = gwp + gwm, gcf = gwp - gwm;
     double gp = 0.0, grho = 0.0, gBx = 0.0, gBy = 0.0, gBz = 0.0;
-    fast_speed_rev(fm, gam, Bx, By, Bz, gcf, gp, grho, gBx, gBy, gBz);
-    fast_speed_rev(fL, gam, L.Bx, L.By, L.Bz, gcfL, gL.p, gL.r, gL.Bx, gL.By, gL.Bz);
-    fast_speed_rev(fR, gam, R.Bx, R.By, R.Bz, gcfR, gR.p, gR.r, gR.Bx, gR.By, gR.Bz);
+    fast_speed_rev<FD>(fm, gam, Bx, By, Bz, gcf, gp, grho, gBx, gBy, gBz);
+    fast_speed_rev<FD>(fL, gam, L.Bx, L.By, L.Bz, gcfL, gL.p, gL.r, gL.Bx, gL.By, gL.Bz);
+    fast_speed_rev<FD>(fR, gam, R.Bx, R.By, R.Bz, gcfR, gR.p, gR.r, gR.Bx, gR.By, gR.Bz);
     gL.r += 0.5 * grho; gR.r += 0.5 * grho;
     gL.p += 0.5 * gp; gR.p += 0.5 * gp;
     gL.u += 0.5 * gu; gR.u += 0.5 * gu;
@@ -951,6 +976,29 @@ __device__ __noinline__ void line_ghost_scatter(const AdjArgs& a, const BlockDes
         adj_scatter<RARE>(a, s, gc);
 }
 
+// The reverse of a flux whose states are out of the branch-free quotients' range.
+struct Flux5 { double q[5]; };
+struct Flux8 { double q[8]; };
+struct FS2 { FS L, R; };
+struct FSm2 { FSm L, R; };
+template <int FLUX>
+__device__ __noinline__ FS2 euler_vjp_out_of_range(GasParams gas, int entropy_fix, FS L, FS R, Flux5 gF) {
+    NumParams P{};
+    P.gas = gas;
+    P.apply_entropy_fix = entropy_fix;
+    FS2 g;
+    if constexpr (FLUX == FLUX_HLLC) hllc_vjp<false>(P, L, R, gF.q, g.L, g.R);
+    else ausmdv_vjp<false>(P, L, R, gF.q, g.L, g.R);
+    return g;
+}
+__device__ __noinline__ FSm2 mhd_vjp_out_of_range(GasParams gas, FSm L, FSm R, Flux8 gF, FSm gL, FSm gR) {
+    NumParams P{};
+    P.gas = gas;
+    FSm2 g{gL, gR};
+    hlle_mhd_vjp<false>(P, L, R, gF.q, g.L, g.R);
+    return g;
+}
+
 // Reverse of the flux of one face for Euler: left and right states in scalar order (normal
 // and tangential velocity, rho, u) with the sound speeds, gF in the face's frame; gl, gr
 // receive the cotangents in the same order, gaL, gaR those of the sound speeds.
@@ -961,8 +1009,15 @@ __device__ __forceinline__ void euler_face_rev(const NumParams& P, const double*
     const FS L{l[3], l[3] * Rg * (l[4] * Cvinv), l[0], l[1], l[2], l[4], aL};
     const FS R{r[3], r[3] * Rg * (r[4] * Cvinv), r[0], r[1], r[2], r[4], aR};
     FS gL, gR;
-    if constexpr (FLUX == FLUX_HLLC) hllc_vjp(P, L, R, gF, gL, gR);
-    else ausmdv_vjp(P, L, R, gF, gL, gR);
+    const double vL[3] = {L.u, L.v, L.w}, vR[3] = {R.u, R.v, R.w};
+    if (flux_in_range<FLUX>(L.r, L.p, L.a, vL, vL, R.r, R.p, R.a, vR, vR)) {
+        if constexpr (FLUX == FLUX_HLLC) hllc_vjp<true>(P, L, R, gF, gL, gR);
+        else ausmdv_vjp<true>(P, L, R, gF, gL, gR);
+    } else {
+        const FS2 g = euler_vjp_out_of_range<FLUX>(P.gas, P.apply_entropy_fix, L, R, Flux5{gF[0], gF[1], gF[2], gF[3], gF[4]});
+        gL = g.L;
+        gR = g.R;
+    }
     // p = rho R (u Cvinv)
     gl[0] = gL.u; gl[1] = gL.v; gl[2] = gL.w;
     gl[3] = gL.r + gL.p * Rg * (l[4] * Cvinv);
@@ -999,7 +1054,16 @@ __device__ __forceinline__ void mhd_face_rev(const AdjArgs& a, const double* l, 
         gL.Bx += 0.5 * gps; gR.Bx += 0.5 * gps;
         gr[8] -= 0.5 * gF[PSI] * ch; gl[8] += 0.5 * gF[PSI] * ch;   // gps / (2 c_h)
     }
-    hlle_mhd_vjp(P, L, R, gF, gL, gR);
+    const double vL[3] = {L.u, L.v, L.w}, vR[3] = {R.u, R.v, R.w};
+    const double BL[3] = {L.Bx, L.By, L.Bz}, BR[3] = {R.Bx, R.By, R.Bz};
+    if (flux_in_range<FLUX_HLLE>(L.r, L.p, 1.0, vL, BL, R.r, R.p, 1.0, vR, BR)) {
+        hlle_mhd_vjp<true>(P, L, R, gF, gL, gR);
+    } else {
+        const FSm2 g = mhd_vjp_out_of_range(P.gas, L, R, Flux8{gF[0], gF[1], gF[2], gF[3], gF[4], gF[5], gF[6], gF[7]},
+                                            gL, gR);
+        gL = g.L;
+        gR = g.R;
+    }
     auto back = [&](const FSm& S, const FSm& gS, double* g) {
         g[0] = gS.u; g[1] = gS.v; g[2] = gS.w;
         g[3] = gS.r + gS.p * Rg * (S.e * Cvinv);   // p = rho R (u Cvinv)
@@ -1008,6 +1072,36 @@ __device__ __forceinline__ void mhd_face_rev(const AdjArgs& a, const double* l, 
     };
     back(L, gL, gl);
     back(R, gR, gr);
+}
+
+// place (prim slot) of scalar s of direction D: face-frame velocity, rho, u, face-frame B, psi
+template <int D, bool MHD>
+__device__ constexpr int scalar_slot(int s) {
+    return s < 3 ? 1 + (D + s) % 3 : s == 3 ? 0 : s == 4 ? 4 : s < 8 ? LineGeo<MHD>::slot(6 + (D + s - 5) % 3) : 8;
+}
+template <int N>
+struct Scalars { double q[N]; };
+// Phase 2 of a cell whose limiters are out of the branch-free reciprocals' range (differences of
+// 1e45 a cell length and more, infinities, NaN): with divisions.  The plus-face states are
+// returned.
+template <int D, bool MHD, bool RARE>
+__device__ __noinline__ Scalars<LineGeo<MHD>::NS> line_recon_out_of_range(const NumParams& P, CellWeights w,
+                                                                          const double* cell, double* minus,
+                                                                          double* recips) {
+    using G = LineGeo<MHD>;
+    constexpr int step = D == 0 ? 1 : 32;
+    Scalars<G::NS> plus;
+    unsigned top = 0u;
+#pragma unroll
+    for (int s = 0; s < G::NS; ++s) {
+        const double* v = cell + scalar_slot<D, MHD>(s) * G::PAD;
+        double qm, rd = 0.0;
+        if (s == 8 && MHD && !P.divergence_cleaning) plus.q[s] = qm = v[0];
+        else cell_recon<RARE, false>(P, w, v[-step], v[0], v[step], qm, plus.q[s], rd, top);
+        minus[s * G::CTA] = qm;
+        recips[s * G::CTA] = rd;
+    }
+    return plus;
 }
 
 template <int D, bool MHD, int FLUX, bool RARE>
@@ -1024,8 +1118,9 @@ __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, doubl
     double* SIN = sm + G::O_IN;
     const NumParams& P = a.P;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // place (prim slot) of scalar s: face-frame velocity, rho, u, face-frame B, psi
-    constexpr int pv[9] = {1 + ax0, 1 + ax1, 1 + ax2, 0, 4, G::slot(6 + ax0), G::slot(6 + ax1), G::slot(6 + ax2), 8};
+    constexpr int pv[9] = {scalar_slot<D, MHD>(0), scalar_slot<D, MHD>(1), scalar_slot<D, MHD>(2),
+                           scalar_slot<D, MHD>(3), scalar_slot<D, MHD>(4), scalar_slot<D, MHD>(5),
+                           scalar_slot<D, MHD>(6), scalar_slot<D, MHD>(7), scalar_slot<D, MHD>(8)};
 
     const long long* off = a.tile_off + D * (a.nblocks + 1);
     int b = 0;
@@ -1103,16 +1198,24 @@ __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, doubl
     bool bad_p = false, bad_m = false;   // e4/onedinterp.d:44-74: the face takes the cell-centre state
     if (active) {
         double qm_r = 1.0, qm_u = 1.0;
+        unsigned top = 0u;
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             const double* v = SP + pv[s] * PAD + pi;
             double qm, rd = 0.0;
             if (s == 8 && !clean) qp[s] = qm = v[0];
-            else cell_recon<RARE>(P, w, v[-step], v[0], v[step], qm, qp[s], rd);
+            else cell_recon<RARE, true>(P, w, v[-step], v[0], v[step], qm, qp[s], rd, top);
             SM[s * T + tid] = qm;
             SR[s * T + tid] = rd;
             if (s == 3) qm_r = qm;
             if (s == 4) qm_u = qm;
+        }
+        if (!P.eps_in_range || !denominators_in_range(top)) {
+            const Scalars<NS> again = line_recon_out_of_range<D, MHD, RARE>(P, w, SP + pi, SM + tid, SR + tid);
+#pragma unroll
+            for (int s = 0; s < NS; ++s) qp[s] = again.q[s];
+            qm_r = SM[3 * T + tid];
+            qm_u = SM[4 * T + tid];
         }
         bad_p = qp[4] <= 0.0 || qp[3] <= 0.0;
         bad_m = qm_u <= 0.0 || qm_r <= 0.0;
