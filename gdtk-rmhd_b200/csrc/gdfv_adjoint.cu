@@ -1123,8 +1123,7 @@ __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, doubl
                            scalar_slot<D, MHD>(6), scalar_slot<D, MHD>(7), scalar_slot<D, MHD>(8)};
 
     const long long* off = a.tile_off + D * (a.nblocks + 1);
-    int b = 0;
-    while (off[b + 1] <= (long long)tile) ++b;
+    const int b = block_of_tile(off, a.nblocks, tile);
     const BlockDesc& B = a.blocks[b];
     const unsigned lt = (unsigned)((long long)tile - off[b]);
     const int n0 = B.n[0], n1 = B.n[1], nD = B.n[D];

@@ -446,7 +446,10 @@ StageArgs stage_args(Context* c) {
 // Cells from which the FP64 stages run as line sweeps (line_sweeps 2): below it they have too
 // few lines to fill the chip.  Both stages, us, sweeps / stage_kernel at its best tiles: 48^3
 // 118 / 92, 64^3 152 / 188, 128x128x64 374 / 518; Orszag-Tang 128x128x4 133 / 120, 256x256x4
-// 240 / 277.
+// 240 / 277.  The line lies at the total, whatever the blocks: lattices of 8,192 blocks of 4^3
+// 1,109 / 2,142, 512 of 8^3 195 / 575, 1,024 of 4x32x4 450 / 1,780 and of 32x4x4 340 / 361, 200
+// of 60x20x2 311 / 334, 8 of 32^3 171 / 187 (default tiles); MHD 8,192 of 4^3 3,147 / 6,126,
+// 512 of 8^3 467 / 1,369.
 constexpr long long kSweepCells = 200000;
 
 // The FP64 line sweeps in the arguments of a launch.

@@ -71,6 +71,19 @@ struct StageArgs {
     double* sweep_part;
 };
 
+// The block that holds tile `tile` in the prefix counts off[0 .. n] of n blocks' tiles.  Halved,
+// not walked: with 8,192 blocks every thread of a sweep read 4,096 offsets first, and a stage
+// took 8.9 ms against 1.0 in stage_kernel.
+__device__ __forceinline__ int block_of_tile(const long long* off, int n, long long tile) {
+    int lo = 0;
+    for (int hi = n; hi - lo > 1;) {
+        const int mid = (lo + hi) >> 1;
+        if (off[mid] <= tile) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
 // Compile-time geometry of the tile and of the shared-memory layout.
 template <class R, bool MHD, int TJ_>
 struct Geo {

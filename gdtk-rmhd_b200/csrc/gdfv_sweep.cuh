@@ -236,12 +236,15 @@ __device__ __forceinline__ void sweep_finish(const StageArgs& A, int stage, cons
 // branch-free quotients' range: minus- and plus-face values.
 template <int N>
 struct Values { double q[N]; };
-template <int NRS, bool MHD, int OPT>
-__device__ __noinline__ Values<2 * NRS> recon_out_of_range(const NumParams& P, const double* w, bool graded,
+template <int NRS, bool MHD, int OPT, int D>
+__device__ __noinline__ Values<2 * NRS> recon_out_of_range(const NumParams& P, const BlockDesc& B, int c,
                                                            Values<NRS> q1, Values<NRS> q0, Values<NRS> q2) {
     Values<2 * NRS> r;
-    if (OPT == 0 && graded) recon_cell_graded_of<double, NRS, MHD, false>(w, P, q1.q, q0.q, q2.q, r.q, r.q + NRS);
-    else recon_cell_of<double, NRS, MHD, OPT, false>(w, P, q1.q, q0.q, q2.q, r.q, r.q + NRS);
+    if (OPT == 0 && B.graded)
+        recon_cell_graded_of<double, NRS, MHD, false>(B.gw[D] + (long long)(c + 1) * GW_N, P, q1.q, q0.q, q2.q, r.q,
+                                                      r.q + NRS);
+    else
+        recon_cell_of<double, NRS, MHD, OPT, false>(B.w[D], P, q1.q, q0.q, q2.q, r.q, r.q + NRS);
     return r;
 }
 
@@ -285,18 +288,15 @@ __global__ void __launch_bounds__(SWEEP_LINES, MHD ? GDFV_MARCH_MINB_MHD : GDFV_
         gather<double, NRS, D>(at, 1, 0, q0);
         gather<double, NRS, D>(hi, 1, 0, q2);
         bool done;
-        const double* gw = nullptr;
-        if (OPT == 0 && B.graded) {
-            gw = B.gw[D] + (long long)(c + 1) * GW_N;
-            done = recon_cell_graded<double, NRS, MHD>(gw, P, q1, q0, q2, qm, qp);
-        } else {
+        if (OPT == 0 && B.graded)
+            done = recon_cell_graded<double, NRS, MHD>(B.gw[D] + (long long)(c + 1) * GW_N, P, q1, q0, q2, qm, qp);
+        else
             done = recon_cell<double, NRS, MHD, OPT>(B.w[D], nullptr, P, q1, q0, q2, qm, qp);
-        }
         if (!done) {
             Values<NRS> v1, v0, v2;
 #pragma unroll
             for (int s = 0; s < NRS; ++s) { v1.q[s] = q1[s]; v0.q[s] = q0[s]; v2.q[s] = q2[s]; }
-            const Values<2 * NRS> r = recon_out_of_range<NRS, MHD, OPT>(P, gw ? gw : B.w[D], gw != nullptr, v1, v0, v2);
+            const Values<2 * NRS> r = recon_out_of_range<NRS, MHD, OPT, D>(P, B, c, v1, v0, v2);
 #pragma unroll
             for (int s = 0; s < NRS; ++s) { qm[s] = r.q[s]; qp[s] = r.q[NRS + s]; }
         }
@@ -333,8 +333,7 @@ __global__ void __launch_bounds__(SWEEP_LINES, MHD ? GDFV_MARCH_MINB_MHD : GDFV_
     if constexpr (D == 0) {
         // a warp's stretch of the stream of slots (rows of n0 + 2: cells -1 .. n0), 32 at a time
         const unsigned full = 0xffffffffu;
-        int b = 0;
-        while (off[b + 1] <= (long long)blockIdx.x) ++b;
+        const int b = block_of_tile(off, A.sweep_blocks, blockIdx.x);
         const BlockDesc& B = A.blocks[b];
         const int n0 = B.n[0], n1 = B.n[1];
         const unsigned n2 = (unsigned)n0 + 2;
@@ -388,8 +387,7 @@ __global__ void __launch_bounds__(SWEEP_LINES, MHD ? GDFV_MARCH_MINB_MHD : GDFV_
         }
     } else {
         double sig_max = 0.0;
-        int blk = 0;
-        while (off[blk + 1] <= (long long)blockIdx.x) ++blk;
+        const int blk = block_of_tile(off, A.sweep_blocks, blockIdx.x);
         const BlockDesc& B = A.blocks[blk];
         const unsigned lt = (unsigned)((long long)blockIdx.x - off[blk]);
         const int n0 = B.n[0], n1 = B.n[1], nD = B.n[D];
