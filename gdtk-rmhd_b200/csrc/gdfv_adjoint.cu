@@ -1598,7 +1598,7 @@ cudaError_t vjp_setup(const AdjView& v, AdjArgs& a, std::vector<long long>& off)
         *v.scratch = nullptr;
         *v.scratch_n = 0;
         *v.scratch_ready = 0;
-        e = cudaMalloc((void**)v.scratch, sizeof(double) * need);
+        e = context_malloc(v.ctx, (void**)v.scratch, sizeof(double) * need);
         if (e != cudaSuccess) return e;
         *v.scratch_n = need;
     }

@@ -30,6 +30,7 @@ std::string noalloc_bad_cell_text(int ctx, long long g);
 
 // What the adjoint (gdfv_adjoint.cu) needs of a context (gdfv_runtime.cu).
 struct AdjView {
+    int ctx;
     int prepared, flux, mhd, precision, nblocks, ninflow, dims;
     long long total;
     const BlockDesc* d_blocks;
@@ -45,6 +46,8 @@ struct AdjView {
 };
 bool adjoint_view(int ctx, AdjView* v);
 void adjoint_set_error(int ctx, const std::string& msg);
+// Device memory for a call on the context (the line sweeps' if there is no other).
+cudaError_t context_malloc(int ctx, void** p, size_t bytes);
 
 // Fixed-dt step chains (gdfv_runtime.cu), for the adjoint's recomputation.
 int steps_dt_prepare(int ctx);

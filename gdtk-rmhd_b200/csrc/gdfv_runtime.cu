@@ -464,6 +464,31 @@ void set_sweeps(const Context* c, StageArgs& A) {
     }
 }
 
+void drop_graphs(Context* c);
+
+// Gives the sweeps' memory back; the stages run in stage_kernel from then on (the same bits).
+void drop_sweeps(Context* c) {
+    cudaStreamSynchronize(c->stream);
+    cudaFree(c->sweep_mem);
+    c->sweep_mem = c->prim[0] = c->prim[1] = c->prim1 = nullptr;
+    c->sweep_part = nullptr;
+    c->d_sweep_off = nullptr;
+    c->sweep = c->prims_valid = false;
+    drop_graphs(c);   // they may hold the sweeps
+}
+
+// Device memory that a call needs.  When there is none left the sweeps give theirs back: what
+// fits beside stage_kernel fits beside them.
+cudaError_t device_malloc(Context* c, void** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !c->sweep_mem) return e;
+    cudaGetLastError();
+    drop_sweeps(c);
+    return cudaMalloc(p, bytes);
+}
+template <class T>
+cudaError_t device_malloc(Context* c, T** p, size_t bytes) { return device_malloc(c, (void**)p, bytes); }
+
 // Arguments of the context's own stepping (gdfv_run, the autotuner, gdfv_time_stages):
 // with the float Euler path or the FP64 sweeps, the primitive buffers of the state buffers it steps
 // (state_parity: which of U[0], U[1] the control record's step parity 0 names).
@@ -536,12 +561,12 @@ cudaError_t enqueue_begin(Context* c) {
 int step_scratch(Context* c) {
     if (c->step_ctl) return 0;
     const size_t nb = c->blocks.size();
-    if (cudaMalloc(&c->step_ctl, sizeof(Control)) != cudaSuccess ||
-        cudaMalloc(&c->step_maxsig, sizeof(unsigned long long) * nb) != cudaSuccess ||
-        cudaMalloc(&c->step_lastsig, sizeof(double) * nb) != cudaSuccess ||
-        cudaMalloc(&c->ch_maxsig, sizeof(unsigned long long) * nb) != cudaSuccess ||
-        cudaMalloc(&c->ch_lastsig, sizeof(double) * nb) != cudaSuccess ||
-        cudaMalloc(&c->ch_bad, sizeof(int)) != cudaSuccess) {
+    if (device_malloc(c, &c->step_ctl, sizeof(Control)) != cudaSuccess ||
+        device_malloc(c, &c->step_maxsig, sizeof(unsigned long long) * nb) != cudaSuccess ||
+        device_malloc(c, &c->step_lastsig, sizeof(double) * nb) != cudaSuccess ||
+        device_malloc(c, &c->ch_maxsig, sizeof(unsigned long long) * nb) != cudaSuccess ||
+        device_malloc(c, &c->ch_lastsig, sizeof(double) * nb) != cudaSuccess ||
+        device_malloc(c, &c->ch_bad, sizeof(int)) != cudaSuccess) {
         fail(c, GDFV_ERR_CUDA, "cudaMalloc of the step scratch failed");
         return 1;
     }
@@ -785,16 +810,18 @@ int sweep_stretch(const Context* c, int d) {
 }
 
 // Buffers and tile offsets of the FP64 line sweeps, when the blocks are large enough for them
-// and device memory holds them beside the state (else stage_kernel takes the stages).
-int prepare_sweeps(Context* c) {
-    if (c->cfg.line_sweeps == 0 || (c->cfg.line_sweeps == 2 && c->total < kSweepCells)) return GDFV_OK;
+// and device memory holds them (else stage_kernel takes the stages): by size (line_sweeps 2)
+// they take at most an eighth of what is free, since the products' and adjoints' scratch and
+// the caller's own arrays come after them.
+void prepare_sweeps(Context* c) {
+    if (c->cfg.line_sweeps == 0 || (c->cfg.line_sweeps == 2 && c->total < kSweepCells)) return;
     const int nb = (int)c->blocks.size();
     std::vector<long long> off(3 * (size_t)(nb + 1), 0);
     for (int d = 0; d < (c->cfg.dims == 3 ? 3 : 2); ++d) {
         c->sweep_cells[d] = d == 0 ? 0 : sweep_stretch(c, d);
         long long* o = off.data() + (size_t)d * (nb + 1);
         for (int b = 0; b < nb; ++b) o[b + 1] = o[b] + sweep_tile_count(c->blocks[b].n, d, c->sweep_cells[d]);
-        if (o[nb] > INT_MAX) return GDFV_OK;
+        if (o[nb] > INT_MAX) return;
         c->sweep_tiles[d] = (int)o[nb];
     }
     const size_t np = c->cfg.mhd ? 10 : 6, cell = sizeof(double) * (size_t)c->total;
@@ -802,13 +829,15 @@ int prepare_sweeps(Context* c) {
     const size_t sizes[5] = {np * cell, np * cell, np * cell, (size_t)c->nq * cell, sizeof(long long) * off.size()};
     size_t at[6] = {0};
     for (int m = 0; m < 5; ++m) at[m + 1] = at[m] + (sizes[m] + 255) / 256 * 256;
+    size_t room = 0, all = 0;
+    if (c->cfg.line_sweeps == 2 && (cudaMemGetInfo(&room, &all) != cudaSuccess || at[5] > room / 8)) return;
     void* mem = nullptr;
     c->sweep = cudaMalloc(&mem, at[5]) == cudaSuccess &&
                cudaMemcpy((char*)mem + at[4], off.data(), sizes[4], cudaMemcpyHostToDevice) == cudaSuccess;
     if (!c->sweep) {
         cudaGetLastError();
         if (mem) cudaFree(mem);
-        return GDFV_OK;
+        return;
     }
     c->sweep_mem = mem;
     c->prim[0] = mem;
@@ -816,7 +845,6 @@ int prepare_sweeps(Context* c) {
     c->prim1 = (char*)mem + at[2];
     c->sweep_part = (double*)((char*)mem + at[3]);
     c->d_sweep_off = (long long*)((char*)mem + at[4]);
-    return GDFV_OK;
 }
 
 int do_prepare(Context* c) {
@@ -1033,10 +1061,6 @@ int do_prepare(Context* c) {
         CK(cudaMalloc(&c->prim[1], pbytes));
         CK(cudaMalloc(&c->prim1, pbytes));
     }
-    if (g.precision == 0) {
-        const int st = prepare_sweeps(c);
-        if (st) return st;
-    }
     c->prims_valid = false;
     if (!geom.empty()) {
         CK(cudaMalloc(&c->d_geom, sizeof(double) * geom.size()));
@@ -1072,6 +1096,7 @@ int do_prepare(Context* c) {
     CK(cudaMalloc(&c->d_bad, sizeof(int)));
     CK(cudaMemset(c->d_maxsig, 0, sizeof(unsigned long long) * c->blocks.size()));
     CK(cudaMemset(c->d_lastsig, 0, sizeof(double) * c->blocks.size()));
+    if (g.precision == 0) prepare_sweeps(c);   // (after all that the context needs)
     c->prepared = true;
     return GDFV_OK;
 }
@@ -1179,10 +1204,19 @@ bool adjoint_view(int ctx, AdjView* v) {
     v->c_h = c->h_ctl ? c->h_ctl->c_h : 0.0;
     v->stream = c->stream;
     v->h_blocks = c->h_blocks;
+    v->ctx = ctx;
     v->scratch = &c->adj_scratch;
     v->scratch_n = &c->adj_scratch_n;
     v->scratch_ready = &c->adj_ready;
     return true;
+}
+
+cudaError_t context_malloc(int ctx, void** p, size_t bytes) {
+    Context* c = get_ctx(ctx);
+    if (!c) return cudaErrorInvalidValue;
+    const cudaError_t e = device_malloc(c, p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 void adjoint_set_error(int ctx, const std::string& msg) {
@@ -1667,13 +1701,13 @@ static int check_ready(Context* c, int blk) {
 static double* io_get(Context* c, long long n) {
     const size_t bytes = sizeof(double) * (size_t)n;
     double* p = nullptr;
-    if (bytes > ((size_t)64 << 20) || c->io_busy.exchange(true)) return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+    if (bytes > ((size_t)64 << 20) || c->io_busy.exchange(true)) return device_malloc(c, &p, bytes) == cudaSuccess ? p : nullptr;
     if (c->io_cap < bytes) {
         double* old = c->io_buf;
         c->io_buf = nullptr;
         c->io_cap = 0;
         if (old) cudaFree(old);
-        if (cudaMalloc(&c->io_buf, bytes) != cudaSuccess) {
+        if (device_malloc(c, &c->io_buf, bytes) != cudaSuccess) {
             c->io_buf = nullptr;
             c->io_busy = false;
             return nullptr;
@@ -1883,7 +1917,7 @@ int upload_tiles(Context* c, const std::vector<TileDesc>& tiles, int n1, int n2,
         if (c->d_tiles) cudaFree(c->d_tiles);
         c->d_tiles = nullptr;
         c->tiles_cap = 0;
-        CK(cudaMalloc(&c->d_tiles, sizeof(TileDesc) * tiles.size()));
+        CK(device_malloc(c, &c->d_tiles, sizeof(TileDesc) * tiles.size()));
         c->tiles_cap = tiles.size();
     }
     CK(cudaMemcpy(c->d_tiles, tiles.data(), sizeof(TileDesc) * tiles.size(), cudaMemcpyHostToDevice));
@@ -1983,7 +2017,7 @@ int autotune(Context* c) {
         int n1 = 0, n2 = 0, n3 = 0, n4 = 0;
         build_tiles(c, kc, tiles, n1, n2, n3, n4);
         int st = upload_tiles(c, tiles, n1, n2, n3, n4);
-        if (st) { cudaEventDestroy(e0); cudaEventDestroy(e1); c->sweep = sweeps; return st; }
+        if (st) { cudaEventDestroy(e0); cudaEventDestroy(e1); c->sweep = sweeps && c->sweep_mem; return st; }
         for (int pers = 1; pers >= 0 && e == cudaSuccess; --pers) {
             const double ms = trial(pers, std::min(best, sweep_ms));
             if (e == cudaSuccess && ms < best) { best = ms; best_kc = kc; best_p = pers; best_w = tw; }
@@ -1993,13 +2027,14 @@ int autotune(Context* c) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    c->sweep = sweeps;
+    c->sweep = sweeps && c->sweep_mem;
     if (e != cudaSuccess) return cuda_fail(c, e, "autotune");
     c->cfg.tile_kchunk = best_kc;
     c->cfg.persistent = best_p;
     c->cfg.tile_width = best_w;
-    c->sweep = sweeps && (sweep_ms < best || c->cfg.line_sweeps == 1);
+    c->sweep = c->sweep && (sweep_ms < best || c->cfg.line_sweeps == 1);
     if (c->sweep) best = sweep_ms;
+    else if (c->sweep_mem) drop_sweeps(c);
     int n1 = 0, n2 = 0, n3 = 0, n4 = 0;
     build_tiles(c, best_kc, tiles, n1, n2, n3, n4);
     int st = upload_tiles(c, tiles, n1, n2, n3, n4);
@@ -2110,7 +2145,7 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
         if (c->d_rec) cudaFree(c->d_rec);
         c->d_rec = nullptr;
         c->rec_cap = 0;
-        CK(cudaMalloc(&c->d_rec, sizeof(double) * ((size_t)nsteps + 1)));
+        CK(device_malloc(c, &c->d_rec, sizeof(double) * ((size_t)nsteps + 1)));
         c->rec_cap = nsteps;
     }
     int* flag = reinterpret_cast<int*>(c->d_rec + nsteps);
@@ -2241,7 +2276,7 @@ int gdfv_residual_jvp(int ctx, const double* U_dev, const double* v_dev, const d
     if (st) return st;
     if (!U_dev || !v_dev || !Jv_dev) return fail(c, GDFV_ERR_ARG, "null pointer");
     const long long n = (long long)c->nq * c->total;
-    if (!c->jvp_scratch) CK(cudaMalloc(&c->jvp_scratch, sizeof(double) * (3 * n + 2 * kJvpSumBlocks)));
+    if (!c->jvp_scratch) CK(device_malloc(c, &c->jvp_scratch, sizeof(double) * (3 * n + 2 * kJvpSumBlocks)));
     double* Up = c->jvp_scratch;
     double* R0 = Up + n;
     double* R1 = R0 + n;
@@ -2357,7 +2392,7 @@ int gdfv_residual_norms(int ctx, double* Linf, double* L2) {
         &per_sm, nq == 10 ? residual_norms_kernel<10> : residual_norms_kernel<5>, kNormThreads, 0));
     const long long want = (c->total + kNormThreads - 1) / kNormThreads;
     const int ncta = (int)std::max(1LL, std::min<long long>(want, (long long)std::min(std::max(per_sm, 1), 8) * n_sm));
-    if (!c->norm_scratch) CK(cudaMalloc(&c->norm_scratch, sizeof(double) * ((size_t)8 * n_sm * 11 + 16)));
+    if (!c->norm_scratch) CK(device_malloc(c, &c->norm_scratch, sizeof(double) * ((size_t)8 * n_sm * 11 + 16)));
     double* out = c->norm_scratch;
     double* partial = c->norm_scratch + 16;
     if (nq == 10)

@@ -63,7 +63,8 @@ int gdfv_context_free(int ctx);
  * fewer lanes idle on blocks whose width is not a multiple of 32), line_sweeps (FP64:
  * 1: each stage as one launch per grid direction on decoded primitives, 0: as one fused
  * launch, 2, the default: by the number of cells; they hold 184 bytes (MHD: 320) a cell
- * more, and are left out when the device has no room for them),
+ * more, by default at most an eighth of the free device memory, are left out when it has no
+ * room for them, and give it back when a later call of the context finds none),
  * autotune (1: the first gdfv_run times the tile k-chunks, both launch forms, both
  * tile widths and the line sweeps, and keeps the fastest).  gdfv_config_get_double also reads
  * tile_kchunk, persistent, tile_width, line_sweeps (after gdfv_prepare: whether the sweeps
