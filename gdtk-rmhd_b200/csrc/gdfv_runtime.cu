@@ -814,7 +814,11 @@ int sweep_stretch(const Context* c, int d) {
 // they take at most an eighth of what is free, since the products' and adjoints' scratch and
 // the caller's own arrays come after them.
 void prepare_sweeps(Context* c) {
-    if (c->cfg.line_sweeps == 0 || (c->cfg.line_sweeps == 2 && c->total < kSweepCells)) return;
+    const Config& g = c->cfg;
+    if (g.line_sweeps == 0) return;
+    // by size, and not where the caller chose a schedule of stage_kernel (the tuner chooses its own)
+    const bool scheduled = (g.tile_kchunk > 0 || g.persistent) && !g.autotune;
+    if (g.line_sweeps == 2 && (c->total < kSweepCells || scheduled)) return;
     const int nb = (int)c->blocks.size();
     std::vector<long long> off(3 * (size_t)(nb + 1), 0);
     for (int d = 0; d < (c->cfg.dims == 3 ? 3 : 2); ++d) {

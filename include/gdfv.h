@@ -62,7 +62,8 @@ int gdfv_context_free(int ctx);
  * cells wide, one row per warp; 16: tiles 16 wide with two rows per warp, which leave
  * fewer lanes idle on blocks whose width is not a multiple of 32), line_sweeps (FP64:
  * 1: each stage as one launch per grid direction on decoded primitives, 0: as one fused
- * launch, 2, the default: by the number of cells; they hold 184 bytes (MHD: 320) a cell
+ * launch, 2, the default: by the number of cells, unless tile_kchunk or persistent asks
+ * for a schedule of the fused launch; they hold 184 bytes (MHD: 320) a cell
  * more, by default at most an eighth of the free device memory, are left out when it has no
  * room for them, and give it back when a later call of the context finds none),
  * autotune (1: the first gdfv_run times the tile k-chunks, both launch forms, both
