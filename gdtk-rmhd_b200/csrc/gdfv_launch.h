@@ -52,8 +52,21 @@ inline int tile_rows_corrector(int precision, bool mhd) {
     return precision == 0 ? (mhd ? TJ_FP64_MHD : TJ_FP64_CORR) : (mhd ? TJ_FP32_MHD_CORR : TJ_FP32_CORR);
 }
 
-// CTAs of the stage kernels resident on one SM (their launch bounds and shared memory).
-inline int tile_ctas_per_sm(int precision, bool mhd) { return precision == 0 ? (mhd ? 1 : 2) : (mhd ? 2 : 3); }
+// CTAs of the stage kernels resident on one SM (their launch bounds; FP64 MHD: their shared memory).
+inline int tile_ctas_per_sm(int precision, bool mhd) {
+    return precision == 0 ? (mhd ? 1 : GDFV_MINB_FP64) : (mhd ? GDFV_MINB_MHD_FP32 : GDFV_MINB_FP32);
+}
+
+// CTAs per SM the FP64 line sweeps are compiled for: 128 registers (Euler), 255 (MHD, no spills;
+// 3 and 4 CTAs spill 0.2 and 0.4 KB: Orszag-Tang 512x512x4 both stages 776 / 830 / 901 us with 2 /
+// 3 / 4, 256x256x4 240 / 268 / 263 us)
+#ifndef GDFV_MARCH_MINB
+#define GDFV_MARCH_MINB 4
+#endif
+#ifndef GDFV_MARCH_MINB_MHD
+#define GDFV_MARCH_MINB_MHD 2
+#endif
+inline int sweep_ctas_per_sm(bool mhd) { return mhd ? GDFV_MARCH_MINB_MHD : GDFV_MARCH_MINB; }
 
 // Options under which the float-flux Euler stages run the kernel on decoded primitives
 // (gdfv_stage_prim.cuh) when the arguments carry primitive buffers (the FP64 form keeps

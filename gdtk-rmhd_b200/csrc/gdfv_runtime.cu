@@ -794,7 +794,7 @@ void exchange_linear(int xm, int face, const int* n, const int* on, int* x) {
 // cells at either end) and the CTAs run T / slots at a time, plus about a third of a wave for
 // the uneven end.  The stretch with the least product, among even cuts of the longest lines.
 int sweep_stretch(const Context* c, int d) {
-    const double slots = (double)c->n_sm * (c->cfg.mhd ? 2 : 4);
+    const double slots = (double)c->n_sm * sweep_ctas_per_sm(c->cfg.mhd);
     int longest = 1;
     for (const HostBlock& hb : c->blocks) longest = std::max(longest, hb.n[d]);
     int best = longest;

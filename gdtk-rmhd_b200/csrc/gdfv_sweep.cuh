@@ -30,21 +30,12 @@
 // The stages read decoded primitives (rho, vel, u, a and for MHD B, psi; SoA), which each
 // stage stores of the state it produces, as the float kernel on decoded primitives does.
 #pragma once
-#include "gdfv_stage.cuh"
+#include "gdfv_launch.h"
 
 namespace gdfv {
 
 constexpr int SWEEP_LINES = 128;   // threads per CTA
 constexpr int SWEEP_WINDOWS = 8;   // windows of 32 slots per warp of the i sweep
-// CTAs per SM the sweeps are compiled for: 128 registers (Euler), 255 (MHD, no spills; 3 and 4
-// CTAs spill 0.2 and 0.4 KB: Orszag-Tang 512x512x4 both stages 776 / 830 / 901 us with 2 / 3 / 4,
-// 256x256x4 240 / 268 / 263 us)
-#ifndef GDFV_MARCH_MINB
-#define GDFV_MARCH_MINB 4
-#endif
-#ifndef GDFV_MARCH_MINB_MHD
-#define GDFV_MARCH_MINB_MHD 2
-#endif
 // Tiles of direction D of a block; cells: those a tile updates along j and k.
 inline long long sweep_tiles(const int* n, int D, int cells) {
     if (D == 0) {   // CTAs of four warps
