@@ -477,14 +477,27 @@ void drop_sweeps(Context* c) {
     drop_graphs(c);   // they may hold the sweeps
 }
 
-// Device memory that a call needs.  When there is none left the sweeps give theirs back: what
-// fits beside stage_kernel fits beside them.
+// Device memory that a call needs.  When there is none left, the buffer kept for flow-state
+// copies and then the sweeps give theirs back: what fits without them fits beside them.
 cudaError_t device_malloc(Context* c, void** p, size_t bytes) {
-    const cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaErrorMemoryAllocation || !c->sweep_mem) return e;
-    cudaGetLastError();
-    drop_sweeps(c);
-    return cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && !c->io_busy.exchange(true)) {   // (in use: a copy's, not spare)
+        double* spare = c->io_buf;
+        c->io_buf = nullptr;
+        c->io_cap = 0;
+        if (spare) {
+            cudaGetLastError();
+            cudaFree(spare);
+            e = cudaMalloc(p, bytes);
+        }
+        c->io_busy = false;
+    }
+    if (e == cudaErrorMemoryAllocation && c->sweep_mem) {
+        cudaGetLastError();
+        drop_sweeps(c);
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 template <class T>
 cudaError_t device_malloc(Context* c, T** p, size_t bytes) { return device_malloc(c, (void**)p, bytes); }

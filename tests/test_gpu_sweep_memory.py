@@ -90,3 +90,22 @@ def test_the_tuner_gives_the_memory_back(tmp_path):
         fakes.fake_room(-1)
     assert left[1] - left[0] >= 184 * total
     """)
+
+
+def test_the_kept_flow_buffer_gives_way(tmp_path):
+    """After flow states have been read, products whose scratch needs the buffer's room."""
+    run_with_fakes(tmp_path, HEAD % "euler" + """
+    def calls(room, flow):
+        fakes.fake_room(room)
+        sim = cases.build_gpu(case, line_sweeps=0)
+        if flow:
+            sim.get_flow(0)
+        check(sim.ctx, sim.L.gdfv_residual_jvp(sim.ctx, _p(U), _p(U), ffi.NULL, 0.0, _p(out[0]), sigma))
+        check(sim.ctx, sim.L.gdfv_residual_vjp(sim.ctx, _p(U), _p(U), _p(out[1]), ffi.NULL))
+        left = fakes.fake_room_left()
+        sim.close()
+        return left
+    least = (1 << 40) - calls(1 << 40, False) - 9 * 8 * total   # without the buffer of the state's way in
+    calls(least + 4096, False)
+    calls(least + 4096, True)
+    """)
