@@ -9,10 +9,11 @@
 // (e4/fvcell.d:586-822) or through a boundary condition (ghost cells).  The VJP
 // runs in three kernels:
 //   1. per cell: decode U -> primitive state P = (rho, v0, v1, v2, u, a);
-//   2. per face: recompute reconstruction and flux from P, then the reverse
-//      sweep; cotangents land on the stencil cells' P (atomics), through the
-//      ghost-cell maps (mirror, copy, xOrder-1 extrapolation, exchange), and on
-//      the fixed inflow states;
+//   2. tiles of grid lines in the three directions, a thread per cell: recompute
+//      reconstruction and the plus face's flux from P, then the reverse of both; a
+//      cell's cotangent, summed over its faces of the direction, is added to its gP
+//      (atomics), through the ghost-cell maps (mirror, copy, xOrder-1
+//      extrapolation, exchange) for ghosts, and to the fixed inflow states;
 //   3. per cell: reverse of decode, gU = (dP/dU)^T gP.
 // Non-smooth points (limiter, clipping, fmax, Mach-number and upwind switches,
 // the entropy fix, |.|) take the branch the primal values took; |x| has
@@ -908,11 +909,12 @@ __device__ void adj_scatter_mhd(const AdjArgs& a, const Src& s, double x, double
 // The transpose of reconstruction and flux along one direction, as tiles of cells of grid
 // lines: one thread per cell, which also takes the face on its plus side.
 //
-// What bounds it: FP64 latency and issue, not bytes.  A thread per face (the form before)
-// evaluates the limiter of each of its two cells forward, again in its reverse, and the two
-// reverses (20 limiters forward and 10 reverse a face for Euler), holds the four stencil
-// cells and their cotangents (168 registers, 12 warps per SM) and scatters all four with
-// atomics.  Per cell there is one limiter a scalar, forward once and reverse once; the
+// What bounds it: FP64 latency and issue, not bytes.  A thread per face would
+// evaluate the limiter of each of its two cells forward, again in its reverse, and the two
+// reverses (20 limiters forward and 10 reverse a face for Euler), hold the four stencil
+// cells and their cotangents (168 registers, 12 warps per SM) and scatter all four with
+// atomics (measured: 817 us a product's faces at 128x128x64 against 385).  Per cell there is
+// one limiter a scalar, forward once and reverse once; the
 // faces' states and the cotangents pass between neighbouring threads in shared memory, and
 // a cell's own cotangent, summed over its faces in this direction, is added once:
 //   1  primitives and W of the tile's cells into shared memory (ghosts by their rules)
@@ -929,10 +931,11 @@ __device__ void adj_scatter_mhd(const AdjArgs& a, const Src& s, double x, double
 #ifndef GDFV_ADJ_J
 #define GDFV_ADJ_J 8
 #endif
-// MHD: 6 layers, 2 CTAs of 192 threads at 168 registers (0.5 KB of spills): 269 us a product
-// on Orszag-Tang 256x256x4 and 249 us at 64^3, against 298 / 263 with 8 layers at 128
-// registers (1.4 KB), 292 / 253 with 4 layers at 3 CTAs and 342 / 262 with 12 at one.  Euler: 8
-// layers, 2 CTAs at 128 registers 456 us at 128x128x64; 6 or 5 layers at 96 registers 461 / 446
+// MHD: 6 layers, 2 CTAs of 192 threads at 168 registers (0.4 KB of spills): 277 us a product
+// on Orszag-Tang 256x256x4 and 256 us at 64^3.  Without the faces' range tests 269 / 249, against
+// 298 / 263 with 8 layers at 128 registers, 292 / 253 with 4 layers at 3 CTAs and 342 / 262
+// with 12 at one.  Euler: 8
+// layers, 2 CTAs at 128 registers 455 us at 128x128x64; 6 or 5 layers at 96 registers 461 / 446
 #ifndef GDFV_ADJ_J_MHD
 #define GDFV_ADJ_J_MHD 6
 #endif
@@ -1635,7 +1638,7 @@ cudaError_t vjp_setup(const AdjView& v, AdjArgs& a, std::vector<long long>& off)
     return cudaSuccess;
 }
 
-// The MHD residual VJP: decode, the face sweep of the three directions, reverse decode.
+// The MHD residual VJP: decode, the line tiles of the three directions, reverse decode.
 cudaError_t enqueue_vjp_mhd(const AdjView& v, const AdjArgs& a, const std::vector<long long>& off) {
     const int nt = 256;
     const unsigned nb_cells = (unsigned)((v.total + nt - 1) / nt);
@@ -1649,7 +1652,7 @@ cudaError_t enqueue_vjp_mhd(const AdjView& v, const AdjArgs& a, const std::vecto
     return cudaGetLastError();
 }
 
-// decode, the three face sweeps (cotangents scattered onto gP) and the reverse decode.
+// decode, the line tiles of the three directions (cotangents added to gP) and the reverse decode.
 cudaError_t enqueue_vjp(const AdjView& v, const AdjArgs& a, const std::vector<long long>& off) {
     const int nt = 256;
     const long long total = v.total;

@@ -445,8 +445,8 @@ StageArgs stage_args(Context* c) {
 
 // Cells from which the FP64 stages run as line sweeps (line_sweeps 2): below it they have too
 // few lines to fill the chip.  Both stages, us, sweeps / stage_kernel at its best tiles: 48^3
-// 118 / 92, 64^3 152 / 188, 128x128x64 374 / 518; Orszag-Tang 128x128x4 133 / 120, 256x256x4
-// 240 / 277.  The line lies at the total, whatever the blocks: lattices of 8,192 blocks of 4^3
+// 118 / 89, 64^3 147 / 176, 128x128x64 367 / 506; Orszag-Tang 128x128x4 130 / 118, 256x256x4
+// 240 / 271.  The line lies at the total, whatever the blocks: lattices of 8,192 blocks of 4^3
 // 1,109 / 2,142, 512 of 8^3 195 / 575, 1,024 of 4x32x4 450 / 1,780 and of 32x4x4 340 / 361, 200
 // of 60x20x2 311 / 334, 8 of 32^3 171 / 187 (default tiles); MHD 8,192 of 4^3 3,147 / 6,126,
 // 512 of 8^3 467 / 1,369.
@@ -639,8 +639,8 @@ void fill_weights(double len, double* w) {
 // time follows (planes per tile + P) x waves: a tile marches its planes one after the
 // other, its prologue costs about P planes (measured 1.5; 3 for the float Euler kernel,
 // whose planes are cheaper), and the tiles run T / slots at a time, plus about a third of
-// a wave for the uneven end.  The chunk with the least product, up to 32, is taken: the
-// old fixed chunk of 32 left most SMs idle on small blocks.  Both stages at 32^3 FP64:
+// a wave for the uneven end.  The chunk with the least product, up to 32, is taken; 32
+// planes a tile leave most SMs idle on small blocks.  Both stages at 32^3 FP64:
 // 563 us with 32 planes a tile, 50 us with 1; 64^3 570 / 153 us (6 planes), 96x80x64 573 /
 // 281 us (12), float 128x128x64 293 / 187 us (12), Orszag-Tang 64x64x32 FP64 886 / 211 us.
 // From about 9 waves on (256^3) it stays 32.
@@ -842,7 +842,7 @@ void prepare_sweeps(Context* c) {
         c->sweep_tiles[d] = (int)o[nb];
     }
     const size_t np = c->cfg.mhd ? 10 : 6, cell = sizeof(double) * (size_t)c->total;
-    // one allocation, parts on 256-byte lines (five took a millisecond more)
+    // one allocation, parts on 256-byte lines (five take a millisecond more)
     const size_t sizes[5] = {np * cell, np * cell, np * cell, (size_t)c->nq * cell, sizeof(long long) * off.size()};
     size_t at[6] = {0};
     for (int m = 0; m < 5; ++m) at[m + 1] = at[m] + (sizes[m] + 255) / 256 * 256;
@@ -1128,8 +1128,8 @@ int read_ctl(Context* c) {
     return GDFV_OK;
 }
 
-// Not waited for: the mirror is pinned, and it is written again only by the host after it has
-// been read back, which the stream orders after this copy.
+// Not waited for: the mirror is pinned, and every call that writes into it again sends it again
+// on the same stream before it launches anything that reads the record.
 int write_ctl(Context* c) {
     CK(cudaMemcpyAsync(c->d_ctl, c->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, c->stream));
     c->ctl_current = true;

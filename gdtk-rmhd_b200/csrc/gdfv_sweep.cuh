@@ -10,14 +10,14 @@
 // three cells, the last plus-face state and the last flux in registers, and a cell's loads are
 // under way (cp.async into the thread's own shared memory) while the cell before it is
 // computed; along i the lanes of a warp are neighbouring cells of a row and exchange states and
-// fluxes by shuffles.  About 830 to 1,240 thread instructions per cell and sweep, 58% issue
-// active at 16 warps, and no re-evaluation but at the ends of stretches.  It pays with memory
-// traffic -- the primitives are read in every sweep and the sums go through memory twice,
+// fluxes by shuffles.  830 to 1,270 thread instructions per cell and sweep, 57 to 63% issue
+// active at 14 warps (16 fit), and no re-evaluation but at the ends of stretches.  It pays with
+// memory traffic -- the primitives are read in every sweep and the sums go through memory twice,
 // 400 to 440 B per cell and stage for Euler against 120 -- which stays below the arithmetic.
 //
-// Measured (both stages, one B200, stage_kernel at its best tiles / sweeps): 256^3 ausmdv 6.58
-// / 4.19 ms, 128x128x64 518 / 374 us, graded hllc 121x85x61 463 / 323 us, Orszag-Tang
-// 256x256x4 277 / 240 us, 512x512x4 1,130 / 782 us.  Tried and slower: the sweeps with one
+// Measured (both stages, one B200, stage_kernel at its best tiles / sweeps): 256^3 ausmdv 6.38
+// / 4.18 ms, 128x128x64 506 / 367 us, graded hllc 121x85x61 449 / 324 us, Orszag-Tang
+// 256x256x4 271 / 240 us, 512x512x4 1,112 / 784 us.  Tried and slower: the sweeps with one
 // thread per cell of a tile, passing states and fluxes in shared memory between barriers
 // (5.07 ms at 256^3 at 24 warps and 80 registers, the same at 16 and 32 warps); the residual
 // sums and U staged in shared memory there (6.3 ms); the walk with its loads in registers

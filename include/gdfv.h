@@ -55,8 +55,10 @@ int gdfv_context_free(int ctx);
  * tile_kchunk.  Doubles: cfl_value, dt_init, dt_max, epsilon_van_albada, R, gamma,
  * divB_damping_length, flowstate_limits_max_velocity, flowstate_limits_max_temp,
  * flowstate_limits_min_temp.  Unknown key or value: GDFV_ERR_ARG.
- * Scheduling integers with no reference counterpart (results do not depend on them):
- * tile_kchunk (planes per tile, 0: up to 32, chosen from the block sizes), persistent (1: each
+ * Scheduling integers with no reference counterpart (FP64 results do not depend on them, the
+ * float-flux form's only to rounding):
+ * tile_kchunk (planes per tile, 0: up to 32, chosen from the block sizes and the device's
+ * SM count), persistent (1: each
  * stage is one resident grid taking the tiles of all blocks from a queue; default 0:
  * one CTA per tile), tile_width (float-flux Euler defaults: 32, the default, tiles 32
  * cells wide, one row per warp; 16: tiles 16 wide with two rows per warp, which leave
