@@ -319,6 +319,9 @@ struct Context {
     int sweep_tiles[3] = {0, 0, 0}, sweep_cells[3] = {0, 0, 0};
     void* sweep_mem = nullptr;         // the allocation that holds prim, prim1, sweep_part and d_sweep_off then
     bool sweep = false;                // the stages run as sweeps (else stage_kernel)
+    // held while launches that pass data in prim1 and sweep_part are put on the stream, so that
+    // another thread's come before or after them all (a graph's launch is one)
+    std::recursive_mutex sweep_mutex;
     bool prims_valid = false;          // prim[parity] holds the primitives of the current state
     long long last_bad_cell = -1;      // global index of the cell the last failure reported (-1: none)
     std::vector<double> h_inflow;      // supersonic-inflow states as uploaded, 9 doubles each (p, T, vel, B, psi)
@@ -468,6 +471,7 @@ void drop_graphs(Context* c);
 
 // Gives the sweeps' memory back; the stages run in stage_kernel from then on (the same bits).
 void drop_sweeps(Context* c) {
+    std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->sweep_mem);
     c->sweep_mem = c->prim[0] = c->prim[1] = c->prim1 = nullptr;
@@ -539,6 +543,7 @@ cudaError_t launch_stage(Context* c, int stage, const StageArgs& A) {
 
 // R(U) of a state anywhere in device memory (the sweeps decode its primitives first).
 cudaError_t launch_residual(Context* c, const double* U, double* R) {
+    std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
     StageArgs A = stage_args(c);
     A.U_in = U;
     A.R_out = R;
@@ -554,6 +559,7 @@ cudaError_t launch_residual(Context* c, const double* U, double* R) {
 // One step of a run, which step_begin_kernel or the step before has begun; it begins the next
 // one unless it is the last slot.
 cudaError_t enqueue_step(Context* c, bool last = false) {
+    std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
     StageArgs A = stage_args_run(c);
     cudaError_t e = launch_stage(c, 1, A);
     if (e != cudaSuccess) return e;
@@ -1997,6 +2003,7 @@ int autotune(Context* c) {
     // above `bound` (a repeat varies by a few per cent, the two launch forms by 10); milliseconds
     const double far = 1.25;
     auto trial = [&](int pers, double bound) {
+        std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
         StageArgs A = stage_args_run(c, parity);
         A.Ubuf[0] = c->U[parity];
         A.Ubuf[1] = c->U[parity ^ 1];
@@ -2468,6 +2475,7 @@ int gdfv_time_stages(int ctx, int reps, double* ms) {
     c->h_ctl->n_fail = 0;
     c->h_ctl->n_invalid1 = 0;
     if (write_ctl(c)) return GDFV_ERR_CUDA;
+    std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
     StageArgs A = stage_args_run(c);
     cudaEvent_t e0, e1, e2;
     CK(cudaEventCreate(&e0));
