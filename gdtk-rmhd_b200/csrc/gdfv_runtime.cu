@@ -2250,6 +2250,7 @@ int gdfv_get_time(int ctx, double* out5, int* step) {
     int st = check_ready(c, -1);
     if (st) return st;
     if (read_ctl(c)) return GDFV_ERR_CUDA;
+    CK(cudaStreamSynchronize(c->stream));   // callers wait here for the calls that only enqueue
     if (out5) {
         out5[0] = c->h_ctl->time; out5[1] = c->h_ctl->dt_global; out5[2] = c->h_ctl->c_h;
         out5[3] = c->h_ctl->cfl_max; out5[4] = c->h_ctl->dt_allow;
@@ -2278,6 +2279,7 @@ int gdfv_set_time(int ctx, double time, int step, double dt_global) {
     c->h_ctl->attempt = 0;
     c->h_ctl->retrying = 0;
     if (write_ctl(c)) return GDFV_ERR_CUDA;
+    CK(cudaStreamSynchronize(c->stream));   // the caller may go on in another stream
     c->signal_valid = false;
     c->prims_valid = false;
     return GDFV_OK;
