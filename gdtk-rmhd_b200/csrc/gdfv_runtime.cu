@@ -2505,6 +2505,7 @@ int gdfv_time_stages(int ctx, int reps, double* ms) {
     *c->h_ctl = saved;
     if (write_ctl(c)) return GDFV_ERR_CUDA;
     c->signal_valid = false;  // the timed corrector stages overwrote the signal maxima
+    c->prims_valid = false;   // a pointer to the state lent before is valid still
     return GDFV_OK;
 }
 
