@@ -320,8 +320,10 @@ struct Context {
     void* sweep_mem = nullptr;         // the allocation that holds prim, prim1, sweep_part and d_sweep_off then
     bool sweep = false;                // the stages run as sweeps (else stage_kernel)
     // held while launches that pass data in prim1 and sweep_part are put on the stream, so that
-    // another thread's come before or after them all (a graph's launch is one)
+    // another thread's come before or after them all (a graph's launch is one), and while the
+    // steps are captured
     std::recursive_mutex sweep_mutex;
+    std::recursive_mutex run_mutex;    // held by a call that steps: nobody takes the sweeps' memory from it
     bool prims_valid = false;          // prim[parity] holds the primitives of the current state
     long long last_bad_cell = -1;      // global index of the cell the last failure reported (-1: none)
     std::vector<double> h_inflow;      // supersonic-inflow states as uploaded, 9 doubles each (p, T, vel, B, psi)
@@ -468,6 +470,7 @@ void set_sweeps(const Context* c, StageArgs& A) {
 }
 
 void drop_graphs(Context* c);
+int build_graph(Context* c);
 
 // Gives the sweeps' memory back; the stages run in stage_kernel from then on (the same bits).
 void drop_sweeps(Context* c) {
@@ -496,10 +499,14 @@ cudaError_t device_malloc(Context* c, void** p, size_t bytes) {
         }
         c->io_busy = false;
     }
-    if (e == cudaErrorMemoryAllocation && c->sweep_mem) {
+    std::unique_lock<std::recursive_mutex> run(c->run_mutex, std::defer_lock);
+    if (e == cudaErrorMemoryAllocation && run.try_lock() && c->sweep_mem) {   // (no other thread's run has them)
         cudaGetLastError();
+        const bool captured = c->graph != nullptr;
         drop_sweeps(c);
         e = cudaMalloc(p, bytes);
+        // (here, not in a later run of a thread beside others that use the stream)
+        if (captured && build_graph(c) != GDFV_OK) drop_graphs(c);
     }
     return e;
 }
@@ -1152,6 +1159,7 @@ void drop_graphs(Context* c) {
 // The step slots of a run, captured once: kGraphSteps of them, and one alone for the
 // tail of a run (a slot past the halt is a no-op, but still launches its kernels).
 int build_graph(Context* c) {
+    std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
     drop_graphs(c);
     for (int n : {kGraphSteps, 1}) {
         cudaGraph_t g = nullptr;
@@ -2094,6 +2102,7 @@ int gdfv_run(int ctx, int max_steps, double max_time, int* steps_taken) {
     if (st) return st;
     if (steps_taken) *steps_taken = 0;
     if (max_steps <= 0) return GDFV_OK;
+    std::lock_guard<std::recursive_mutex> run(c->run_mutex);
     if (!c->signal_valid) {
         if ((st = scan_signal(c)) != GDFV_OK) return st;
     }
@@ -2155,6 +2164,7 @@ int gdfv_run_record(int ctx, int nsteps, double* const* states_dev, double* cons
     if (st) return st;
     if (nsteps < 1 || !states_dev || !preds_dev || !dts)
         return fail(c, GDFV_ERR_ARG, "gdfv_run_record needs nsteps >= 1, the two pointer arrays and dts");
+    std::lock_guard<std::recursive_mutex> run(c->run_mutex);
     if (!c->signal_valid) {
         if ((st = scan_signal(c)) != GDFV_OK) return st;
     }
@@ -2290,6 +2300,7 @@ int gdfv_residual(int ctx, const double* U_dev, double* R_dev) {
     int st = check_ready(c, -1);
     if (st) return st;
     if (!U_dev || !R_dev) return fail(c, GDFV_ERR_ARG, "null pointer");
+    std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
     CK(launch_residual(c, U_dev, R_dev));
     CK(cudaStreamSynchronize(c->stream));
     return GDFV_OK;
@@ -2303,6 +2314,7 @@ int gdfv_residual_jvp(int ctx, const double* U_dev, const double* v_dev, const d
     if (!U_dev || !v_dev || !Jv_dev) return fail(c, GDFV_ERR_ARG, "null pointer");
     const long long n = (long long)c->nq * c->total;
     if (!c->jvp_scratch) CK(device_malloc(c, &c->jvp_scratch, sizeof(double) * (3 * n + 2 * kJvpSumBlocks)));
+    std::lock_guard<std::recursive_mutex> lk(c->sweep_mutex);
     double* Up = c->jvp_scratch;
     double* R0 = Up + n;
     double* R1 = R0 + n;
@@ -2465,6 +2477,7 @@ int gdfv_time_stages(int ctx, int reps, double* ms) {
     int st = check_ready(c, -1);
     if (st) return st;
     if (reps < 1 || !ms) return fail(c, GDFV_ERR_ARG, "bad argument");
+    std::lock_guard<std::recursive_mutex> run(c->run_mutex);
     if (!c->signal_valid && (st = scan_signal(c)) != GDFV_OK) return st;
     if ((st = ensure_prims(c)) != GDFV_OK) return st;
     if (read_ctl(c)) return GDFV_ERR_CUDA;

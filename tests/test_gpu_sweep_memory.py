@@ -109,3 +109,36 @@ def test_the_kept_flow_buffer_gives_way(tmp_path):
     calls(least + 4096, False)
     calls(least + 4096, True)
     """)
+
+
+def test_memory_is_not_taken_from_a_run_of_another_thread(tmp_path):
+    """Products that find no memory while another thread steps the context: they fail or, between
+    runs, take the sweeps' memory; the run's states are those of a run alone."""
+    run_with_fakes(tmp_path, HEAD % "euler" + """
+    import threading
+    alone, sim = cases.build_gpu(case), cases.build_gpu(case)
+    assert sim.option("line_sweeps") == 1
+    for s in (alone, sim):
+        assert s.run(max_step=1) == 1   # the steps are captured
+    U.copy_(torch.from_numpy(sim.get_conserved(0)))
+    torch.cuda.synchronize()
+    errors = []
+    def steps():
+        try:
+            for _ in range(10):
+                assert sim.run(max_step=17) == 17
+        except Exception as e:
+            errors.append(repr(e))
+    fakes.fake_room(0)
+    t = threading.Thread(target=steps)
+    t.start()
+    refused = 0
+    while t.is_alive():
+        refused += sim.L.gdfv_residual_jvp(sim.ctx, _p(U), _p(U), ffi.NULL, 1e-3, _p(out[0]), sigma) != 0
+    t.join()
+    fakes.fake_room(-1)
+    assert not errors, errors
+    print("refused", refused, "sweeps", sim.option("line_sweeps"))
+    assert alone.run(max_step=170) == 170
+    assert np.array_equal(alone.get_conserved(0), sim.get_conserved(0))
+    """)
