@@ -913,7 +913,7 @@ __device__ void adj_scatter_mhd(const AdjArgs& a, const Src& s, double x, double
 // evaluate the limiter of each of its two cells forward, again in its reverse, and the two
 // reverses (20 limiters forward and 10 reverse a face for Euler), hold the four stencil
 // cells and their cotangents (168 registers, 12 warps per SM) and scatter all four with
-// atomics (measured: 817 us a product's faces at 128x128x64 against 385).  Per cell there is
+// atomics (measured: 817 us a product's faces at 128x128x64 against 388).  Per cell there is
 // one limiter a scalar, forward once and reverse once; the
 // faces' states and the cotangents pass between neighbouring threads in shared memory, and
 // a cell's own cotangent, summed over its faces in this direction, is added once:
@@ -931,11 +931,11 @@ __device__ void adj_scatter_mhd(const AdjArgs& a, const Src& s, double x, double
 #ifndef GDFV_ADJ_J
 #define GDFV_ADJ_J 8
 #endif
-// MHD: 6 layers, 2 CTAs of 192 threads at 168 registers (0.4 KB of spills): 277 us a product
-// on Orszag-Tang 256x256x4 and 256 us at 64^3.  Without the faces' range tests 269 / 249, against
+// MHD: 6 layers, 2 CTAs of 192 threads at 168 registers (0.4 KB of spills): 272 us a product
+// on Orszag-Tang 256x256x4 and 251 us at 64^3.  Without the faces' range tests 269 / 249, against
 // 298 / 263 with 8 layers at 128 registers, 292 / 253 with 4 layers at 3 CTAs and 342 / 262
 // with 12 at one.  Euler: 8
-// layers, 2 CTAs at 128 registers 455 us at 128x128x64; 6 or 5 layers at 96 registers 461 / 446
+// layers, 2 CTAs at 128 registers 454 us at 128x128x64; 6 or 5 layers at 96 registers 461 / 446
 #ifndef GDFV_ADJ_J_MHD
 #define GDFV_ADJ_J_MHD 6
 #endif
@@ -979,48 +979,18 @@ __device__ __noinline__ void line_ghost_scatter(const AdjArgs& a, const BlockDes
         adj_scatter<RARE>(a, s, gc);
 }
 
-// The reverse of a flux whose states are out of the branch-free quotients' range.
-struct Flux5 { double q[5]; };
-struct Flux8 { double q[8]; };
-struct FS2 { FS L, R; };
-struct FSm2 { FSm L, R; };
-template <int FLUX>
-__device__ __noinline__ FS2 euler_vjp_out_of_range(GasParams gas, int entropy_fix, FS L, FS R, Flux5 gF) {
-    NumParams P{};
-    P.gas = gas;
-    P.apply_entropy_fix = entropy_fix;
-    FS2 g;
-    if constexpr (FLUX == FLUX_HLLC) hllc_vjp<false>(P, L, R, gF.q, g.L, g.R);
-    else ausmdv_vjp<false>(P, L, R, gF.q, g.L, g.R);
-    return g;
-}
-__device__ __noinline__ FSm2 mhd_vjp_out_of_range(GasParams gas, FSm L, FSm R, Flux8 gF, FSm gL, FSm gR) {
-    NumParams P{};
-    P.gas = gas;
-    FSm2 g{gL, gR};
-    hlle_mhd_vjp<false>(P, L, R, gF.q, g.L, g.R);
-    return g;
-}
-
 // Reverse of the flux of one face for Euler: left and right states in scalar order (normal
 // and tangential velocity, rho, u) with the sound speeds, gF in the face's frame; gl, gr
 // receive the cotangents in the same order, gaL, gaR those of the sound speeds.
-template <int FLUX>
+template <int FLUX, bool FD>
 __device__ __forceinline__ void euler_face_rev(const NumParams& P, const double* l, double aL, const double* r, double aR,
                                                const double* gF, double* gl, double& gaL, double* gr, double& gaR) {
     const double Rg = P.gas.R, Cvinv = P.gas.Cvinv;
     const FS L{l[3], l[3] * Rg * (l[4] * Cvinv), l[0], l[1], l[2], l[4], aL};
     const FS R{r[3], r[3] * Rg * (r[4] * Cvinv), r[0], r[1], r[2], r[4], aR};
     FS gL, gR;
-    const double vL[3] = {L.u, L.v, L.w}, vR[3] = {R.u, R.v, R.w};
-    if (flux_in_range<FLUX>(L.r, L.p, L.a, vL, vL, R.r, R.p, R.a, vR, vR)) {
-        if constexpr (FLUX == FLUX_HLLC) hllc_vjp<true>(P, L, R, gF, gL, gR);
-        else ausmdv_vjp<true>(P, L, R, gF, gL, gR);
-    } else {
-        const FS2 g = euler_vjp_out_of_range<FLUX>(P.gas, P.apply_entropy_fix, L, R, Flux5{gF[0], gF[1], gF[2], gF[3], gF[4]});
-        gL = g.L;
-        gR = g.R;
-    }
+    if constexpr (FLUX == FLUX_HLLC) hllc_vjp<FD>(P, L, R, gF, gL, gR);
+    else ausmdv_vjp<FD>(P, L, R, gF, gL, gR);
     // p = rho R (u Cvinv)
     gl[0] = gL.u; gl[1] = gL.v; gl[2] = gL.w;
     gl[3] = gL.r + gL.p * Rg * (l[4] * Cvinv);
@@ -1036,6 +1006,7 @@ __device__ __forceinline__ void euler_face_rev(const NumParams& P, const double*
 // the conserved quantities (face frame), psi and divB included.  F[divB] = (BxR - BxL)/2 and
 // the GLM terms (fluxcalc.d:139-150, with the reference's third term added to F[xB] under
 // glm_reference_indexing) with c_h held fixed, then hlle.
+template <bool FD>
 __device__ __forceinline__ void mhd_face_rev(const AdjArgs& a, const double* l, const double* r, const double* gF,
                                              double* gl, double* gr) {
     const NumParams& P = a.P;
@@ -1057,16 +1028,7 @@ __device__ __forceinline__ void mhd_face_rev(const AdjArgs& a, const double* l, 
         gL.Bx += 0.5 * gps; gR.Bx += 0.5 * gps;
         gr[8] -= 0.5 * gF[PSI] * ch; gl[8] += 0.5 * gF[PSI] * ch;   // gps / (2 c_h)
     }
-    const double vL[3] = {L.u, L.v, L.w}, vR[3] = {R.u, R.v, R.w};
-    const double BL[3] = {L.Bx, L.By, L.Bz}, BR[3] = {R.Bx, R.By, R.Bz};
-    if (flux_in_range<FLUX_HLLE>(L.r, L.p, 1.0, vL, BL, R.r, R.p, 1.0, vR, BR)) {
-        hlle_mhd_vjp<true>(P, L, R, gF, gL, gR);
-    } else {
-        const FSm2 g = mhd_vjp_out_of_range(P.gas, L, R, Flux8{gF[0], gF[1], gF[2], gF[3], gF[4], gF[5], gF[6], gF[7]},
-                                            gL, gR);
-        gL = g.L;
-        gR = g.R;
-    }
+    hlle_mhd_vjp<FD>(P, L, R, gF, gL, gR);
     auto back = [&](const FSm& S, const FSm& gS, double* g) {
         g[0] = gS.u; g[1] = gS.v; g[2] = gS.w;
         g[3] = gS.r + gS.p * Rg * (S.e * Cvinv);   // p = rho R (u Cvinv)
@@ -1105,6 +1067,49 @@ __device__ __noinline__ Scalars<LineGeo<MHD>::NS> line_recon_out_of_range(const 
         recips[s * G::CTA] = rd;
     }
     return plus;
+}
+
+// Cotangent of a face's flux in its frame, from W of the cells to the left and right (at wl and wr).
+template <int D, bool MHD>
+__device__ __forceinline__ void face_cotangent(const double* wl, const double* wr, double AVl, double AVr, double* gF) {
+    constexpr int T = LineGeo<MHD>::CTA;
+#pragma unroll
+    for (int q = 0; q < LineGeo<MHD>::NQ; ++q) {
+        // momentum and B components in the order normal, tangents
+        const int qg = q >= 1 && q <= 3 ? 1 + (D + q - 1) % 3 : (MHD && q >= 5 && q <= 7 ? 5 + (D + q - 5) % 3 : q);
+        gF[q] = AVr * wr[qg * T] - AVl * wl[qg * T];
+    }
+}
+// Phase 3 of a face whose states l and r (minus-face state of the cell to the right, replaced by
+// its cotangent) are out of the branch-free reciprocals' range: with divisions.  The cotangents of
+// l and, after them, of its sound speed are returned; sa: the sound speeds of the cells.  It reads W
+// and r again: handed over in registers they cost a product 4 to 5 us (hllc 470 against 465,
+// MHD 277 against 272).
+template <int D, bool MHD, int FLUX>
+__device__ __noinline__ Scalars<LineGeo<MHD>::NS + 1> line_face_out_of_range(const AdjArgs& a, Scalars<LineGeo<MHD>::NS> l,
+                                                                             double AVl, double AVr, const double* wl,
+                                                                             double* minus, double* sa) {
+    using G = LineGeo<MHD>;
+    constexpr int step = D == 0 ? 1 : 32;
+    Scalars<G::NS + 1> out;
+    double gF[G::NQ], r[G::NS], gr[G::NS];
+    face_cotangent<D, MHD>(wl, wl + step, AVl, AVr, gF);
+#pragma unroll
+    for (int s = 0; s < G::NS; ++s) r[s] = minus[s * G::CTA];
+    out.q[G::NS] = 0.0;
+    if constexpr (MHD)
+        mhd_face_rev<false>(a, l.q, r, gF, out.q, gr);
+    else
+        euler_face_rev<FLUX, false>(a.P, l.q, sa[0], r, sa[step], gF, out.q, out.q[G::NS], gr, sa[G::CTA + step]);
+#pragma unroll
+    for (int s = 0; s < G::NS; ++s) minus[s * G::CTA] = gr[s];
+    return out;
+}
+// flux_in_range of the states l and r of a face in scalar order
+template <int FLUX>
+__device__ __forceinline__ bool face_in_range(const GasParams& gas, const double* l, double aL, const double* r, double aR) {
+    const double pL = l[3] * gas.R * (l[4] * gas.Cvinv), pR = r[3] * gas.R * (r[4] * gas.Cvinv);
+    return flux_in_range<FLUX>(l[3], pL, aL, l, l + 5, r[3], pR, aR, r, r + 5);
 }
 
 template <int D, bool MHD, int FLUX, bool RARE>
@@ -1252,13 +1257,6 @@ __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, doubl
             AVl = Af * rcp(threeD ? Ll[0] * Ll[1] * Ll[2] : Ll[0] * Ll[1]) * a.w_scale;
         }
         const int nb = tid + step;   // the cell to the right
-        double gF[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            // the face's frame: momentum and B components in the order normal, tangents
-            const int qg = q >= 1 && q <= 3 ? 1 + (D + q - 1) % 3 : (MHD && q >= 5 && q <= 7 ? 5 + (D + q - 5) % 3 : q);
-            gF[q] = AVr * SW[qg * T + nb] - AVl * SW[qg * T + tid];
-        }
         const int bface = c == -1 ? 2 * D : (c == nD - 1 ? 2 * D + 1 : -1);
         bool simple = false;
         if constexpr (RARE && !MHD) simple = bface >= 0 && B.bc_type[bface] == BC_SIMPLE_FLUX;
@@ -1267,6 +1265,8 @@ __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, doubl
                 // OutFlowBC_SimpleFlux (boundary_flux_effect.d:504-645): the boundary face's flux is
                 // the interior cell's outflow flux, or only its pressure on a closed face
                 const int at = pi + ((bface & 1) ? 0 : step);
+                double gF[NQ];
+                face_cotangent<D, MHD>(SW + tid, SW + nb, AVl, AVr, gF);
                 double gg[5] = {gF[MASS], 0.0, 0.0, 0.0, gF[TOTENERGY]}, cs[6], gs[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
                 gg[1 + ax0] = gF[1]; gg[1 + ax1] = gF[2]; gg[1 + ax2] = gF[3];
                 for (int s = 0; s < 5; ++s) cs[s] = SP[s * PAD + at];
@@ -1280,18 +1280,27 @@ __device__ __forceinline__ void line_tile(const AdjArgs& a, unsigned tile, doubl
             }
         }
         if (!simple) {
-            double r[NS], gl[NS], gr[NS];
+            double r[NS];
 #pragma unroll
             for (int s = 0; s < NS; ++s) r[s] = SM[s * T + nb];
-            if constexpr (MHD) {
-                mhd_face_rev(a, qp, r, gF, gl, gr);
-            } else {
-                double gaR;
-                euler_face_rev<FLUX>(P, qp, SA[tid], r, SA[nb], gF, gl, ga, gr, gaR);
-                SA[T + nb] = gaR;
-            }
+            if (face_in_range<FLUX>(P.gas, qp, MHD ? 1.0 : SA[tid], r, MHD ? 1.0 : SA[nb])) {
+                double gF[NQ], gl[NS], gr[NS];
+                face_cotangent<D, MHD>(SW + tid, SW + nb, AVl, AVr, gF);
+                if constexpr (MHD)
+                    mhd_face_rev<true>(a, qp, r, gF, gl, gr);
+                else
+                    euler_face_rev<FLUX, true>(P, qp, SA[tid], r, SA[nb], gF, gl, ga, gr, SA[T + nb]);
 #pragma unroll
-            for (int s = 0; s < NS; ++s) { qp[s] = gl[s]; SM[s * T + nb] = gr[s]; }
+                for (int s = 0; s < NS; ++s) { qp[s] = gl[s]; SM[s * T + nb] = gr[s]; }
+            } else {
+                Scalars<NS> l;
+#pragma unroll
+                for (int s = 0; s < NS; ++s) l.q[s] = qp[s];
+                const Scalars<NS + 1> g = line_face_out_of_range<D, MHD, FLUX>(a, l, AVl, AVr, SW + tid, SM + nb, SA + tid);
+#pragma unroll
+                for (int s = 0; s < NS; ++s) qp[s] = g.q[s];
+                ga = g.q[NS];
+            }
         }
     } else {
 #pragma unroll
